@@ -520,12 +520,12 @@ spt_status spt_scene_create(spt_context* ctx, const spt_scene_desc* d, const spt
                     const uint32_t type = d->prim_type[slot_prim[rk]];
                     if (type == SPT_PRIM_SPHERE) {
                         wtri[3 * k] = make_float4(r[0].x, r[0].y, r[0].z, bits_f(rk));
-                        wtri[3 * k + 1] = make_float4(0.0f, 0.0f, 0.0f, bits_f(type));
-                        wtri[3 * k + 2] = make_float4(r[1].x, 0.0f, 0.0f, r[1].w);
+                        wtri[3 * k + 1] = make_float4(0.0f, 0.0f, 0.0f, r[0].w);
+                        wtri[3 * k + 2] = make_float4(r[1].x, 0.0f, 0.0f, bits_f(slot_leaf[rk] | 0x80000000u));
                     } else {
                         wtri[3 * k] = make_float4(r[0].x, r[0].y, r[0].z, bits_f(rk));
-                        wtri[3 * k + 1] = make_float4(r[1].x, r[1].y, r[1].z, bits_f(type));
-                        wtri[3 * k + 2] = make_float4(r[2].x, r[2].y, r[2].z, r[1].w);  // leaf id
+                        wtri[3 * k + 1] = make_float4(r[1].x, r[1].y, r[1].z, r[0].w);  // primitive id
+                        wtri[3 * k + 2] = make_float4(r[2].x, r[2].y, r[2].z, bits_f(slot_leaf[rk]));
                     }
                 }
             });

@@ -175,57 +175,47 @@ __global__ void __launch_bounds__(256) k_extend(Wave W, const Counters* __restri
     }
 }
 
+// The iteration's live slots as the persistent extend kernel takes them.  With one scene (MANY false)
+// its pointers stay in the constant bank; with a batch every lane holds its path's, by value, so that
+// they are not reloaded from the job table at every node.
+template <bool MANY>
+struct PathRays {
+    const DevScene& S;
+    const Wave& W;
+    const PathBuf& cur;
+    float4* hits;
+    const DevScene* mine;
+    WideScene ws;
+    __device__ __forceinline__ void load(uint32_t i, V3& o, V3& d) {
+        if (MANY) {
+            mine = &W.jobs[__float_as_uint(cur.b[i].w) >> 16].S;
+            ws = wide_scene(*mine);
+        }
+        o = f3v(cur.o[i]);
+        d = f3v(cur.d[i]);
+    }
+    __device__ __forceinline__ const float* root_min() const { return MANY ? mine->root_min : S.root_min; }
+    __device__ __forceinline__ const float* root_max() const { return MANY ? mine->root_max : S.root_max; }
+    __device__ __forceinline__ WideScene scene() const { return MANY ? ws : wide_scene(S); }
+    __device__ __forceinline__ void store(uint32_t i, float t, uint32_t prim, float u, float v) {
+        hits[i] = make_float4(t, __uint_as_float(prim), u, v);
+    }
+};
+
 // Persistent extend: lanes take live slots from the iteration's counter as their rays finish.
-// DEPTH: the lane's traversal stack depth (tune.stack); W.stack_limit may hold it lower.
-template <int DEPTH>
-__global__ void __launch_bounds__(128) k_extend_df(Wave W, Counters* __restrict__ ctr, PathBuf cur,
+// DEPTH: the lane's traversal stack depth (tune.stack); W.stack_limit may hold it lower.  MANY: the
+// batch's jobs are of several scenes (S is the one scene otherwise).  Blocks per SM by measurement:
+// the layered scene 19.1 ms at 8 and 19.4 at 7 (72 registers), the box level; the batch, whose lanes
+// hold their scene's pointers, 20.0 ms at 7 and 20.9 at 8.
+template <int DEPTH, bool MANY>
+__global__ void __launch_bounds__(128, MANY ? 7 : 8) k_extend_df(const __grid_constant__ Wave W, const __grid_constant__ DevScene S,
+                                                   Counters* __restrict__ ctr, const __grid_constant__ PathBuf cur,
                                                    float4* __restrict__ hits, uint32_t* status) {
+    __shared__ WarpQueue q[4];
     const Counters c = *ctr;
     const uint32_t n = c.n_alive + n_new_paths(W, c);
-    const uint32_t lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    const int limit = static_cast<int>(W.stack_limit);
-    WideTraversalT<true, DEPTH> tr;
-    // the lane's scene, held by value: the fields the traversal reads stay in registers instead of
-    // being reloaded from the job table at every node
-    DevScene S{};
-    bool active = false, exhausted = false;
-    unsigned long long mine = 0, pool = 0, pool_end = 0;
-    for (;;) {
-        const unsigned need = __ballot_sync(0xFFFFFFFFu, !active && !exhausted);
-        if (need) {
-            const uint32_t cnt = __popc(need), rank = __popc(need & lt);
-            const unsigned long long have = pool_end - pool;
-            unsigned long long fresh = 0;
-            if (have < cnt) {
-                if (lane == 0) fresh = atomicAdd(&ctr->fetch, static_cast<unsigned long long>(kChunk));
-                fresh = __shfl_sync(0xFFFFFFFFu, fresh, 0);
-            }
-            if (!active && !exhausted) {
-                mine = rank < have ? pool + rank : fresh + (rank - have);
-                if (mine >= n) {
-                    exhausted = true;
-                } else {
-                    S = W.jobs[__float_as_uint(cur.b[mine].w) >> 16].S;
-                    active = tr.start(S, f3v(cur.o[mine]), f3v(cur.d[mine]));
-                    if (!active) hits[mine] = hit_record(S, tr.h);
-                }
-            }
-            if (have < cnt) {
-                pool = fresh + (cnt - have);
-                pool_end = fresh + kChunk;
-            } else {
-                pool += cnt;
-            }
-        }
-        if (__all_sync(0xFFFFFFFFu, !active && exhausted)) break;
-        if (active && !tr.step(S, status, limit)) {
-            if (tr.finish(S)) {
-                hits[mine] = hit_record(S, tr.h);
-                active = false;
-            }
-        }
-    }
+    PathRays<MANY> src{S, W, cur, hits, &S, wide_scene(S)};
+    persistent_trace<DEPTH, false>(q[threadIdx.x >> 5], src, n, &ctr->fetch, static_cast<int>(W.stack_limit), status);
 }
 
 __device__ __forceinline__ void splat(const PtJob& J, uint32_t pix, V3 L) {
@@ -679,7 +669,16 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
     const unsigned g_gen = static_cast<unsigned>(std::min<uint64_t>((cap + 255) / 256, 8ull * sms));
     const unsigned g_ext = static_cast<unsigned>(std::min<uint64_t>((cap + eb - 1) / eb, 16ull * sms * 128 / eb));
     const unsigned g_shd = static_cast<unsigned>(std::min<uint64_t>((cap + sb - 1) / sb, 16ull * sms * 128 / sb));
-    auto ext_df = depth == 16 ? k_extend_df<16> : depth == 24 ? k_extend_df<24> : k_extend_df<32>;
+    // one scene for the whole batch: its pointers go to the extend kernel as a parameter
+    bool many = false;
+    const DevScene* one = nullptr;
+    for (const PtJob& J : jobs) {
+        if (!J.total) continue;
+        if (!one) one = &J.S;
+        else many |= std::memcmp(one, &J.S, sizeof(DevScene)) != 0;
+    }
+    auto ext_df = many ? (depth == 16 ? k_extend_df<16, true> : depth == 24 ? k_extend_df<24, true> : k_extend_df<32, true>)
+                       : (depth == 16 ? k_extend_df<16, false> : depth == 24 ? k_extend_df<24, false> : k_extend_df<32, false>);
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ext_df, 128, 0);
     const unsigned g_df = static_cast<unsigned>(sms * std::max(1, per_sm));
@@ -697,7 +696,7 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
             PathBuf& cur = it ? B : A;
             PathBuf& nxt = it ? A : B;
             k_generate<<<g_gen, 256, 0, ctx->stream>>>(W, d_ctr, cur);
-            if (trav == 2) ext_df<<<g_df, 128, 0, ctx->stream>>>(W, d_ctr, cur, hits, ctx->d_status);
+            if (trav == 2) ext_df<<<g_df, 128, 0, ctx->stream>>>(W, *one, d_ctr, cur, hits, ctx->d_status);
             else if (trav == 1) k_extend<1><<<g_ext, eb, 0, ctx->stream>>>(W, d_ctr, cur, hits, ctx->d_status);
             else k_extend<0><<<g_ext, eb, 0, ctx->stream>>>(W, d_ctr, cur, hits, ctx->d_status);
             const uint32_t* order = nullptr;

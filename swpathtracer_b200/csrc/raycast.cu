@@ -5,6 +5,7 @@
 //   k_raycast     camera ray generation fused with the query and the pixel value of one
 //                 ray-caster mode (integrators/raycaster.h:62-99 + normal_raycaster.cpp:19-31,
 //                 depth_raycaster.cpp:36-48, int_test_count_raycaster.cpp:75-85)
+#include <algorithm>
 #include <cstring>
 #include <limits>
 
@@ -35,54 +36,65 @@ __device__ __forceinline__ void load_ray(const float* __restrict__ rays, uint64_
     }
 }
 
+// Rays and hits of the persistent kernels.  Rays are read and hits written once, with the evict-first
+// (streaming) cache hint, so the ray and hit streams (48 B per ray, 768 MB per 2^24 rays) push less of
+// the scene out of L2: +1 %.  ORDERED: the k-th ray taken is order[k] (ray_order.cu) and its hit goes
+// to place k, so that neighbouring lanes write neighbouring hits (scattered 16-byte stores cost
+// partial-sector writes in DRAM).
+template <int STRIDE, bool ORDERED>
+struct RayBatch {
+    const DevScene& S;
+    const float* rays;
+    const uint32_t* order;
+    spt_hit* hits;
+    __device__ __forceinline__ void load(uint32_t i, V3& o, V3& d) {
+        load_ray<STRIDE, true>(rays, ORDERED ? __ldg(order + i) : i, o, d);
+    }
+    __device__ __forceinline__ const float* root_min() const { return S.root_min; }
+    __device__ __forceinline__ const float* root_max() const { return S.root_max; }
+    __device__ __forceinline__ WideScene scene() const { return wide_scene(S); }
+    __device__ __forceinline__ void store(uint32_t i, float t, uint32_t prim, float u, float v) {
+        __stcs(reinterpret_cast<float4*>(hits + i), make_float4(t, __uint_as_float(prim), u, v));
+    }
+};
+
 // Persistent variant: wide traversal, lanes refilled from a global ray counter (traverse_wide.cuh).
-// 10 blocks of 128 per SM (at most 48 registers): 40 resident warps to hide the node-fetch latency.
-// Rays are read and hits written once, with the evict-first (streaming) cache hint, so the ray and
-// hit streams (48 B per ray, 768 MB per 2^24 rays) push less of the scene out of L2: +1 %.
+// 8 blocks of 128 per SM (at most 64 registers): on 2^24 incoherent rays 3.86 ms a step against 4.22 at
+// 10 blocks (48 registers, 150 bytes spilled), 3.93 at 7 and 4.22 at 6.
 template <int STRIDE>
-__global__ void __launch_bounds__(kBlock, 10) k_intersect_df(DevScene S, const float* __restrict__ rays, uint64_t n,
+__global__ void __launch_bounds__(kBlock, 8) k_intersect_df(const __grid_constant__ DevScene S,
+                                                         const float* __restrict__ rays, uint32_t n,
                                                          spt_hit* __restrict__ hits, uint32_t* status,
                                                          unsigned long long* next) {
-    persistent_trace(
-        S, n, next, status, [&](uint64_t i, V3& o, V3& d) { load_ray<STRIDE, true>(rays, i, o, d); },
-        [&](uint64_t i, const Hit1& h) {
-            __stcs(reinterpret_cast<float4*>(hits + i),
-                   make_float4(h.t, __uint_as_float(h.found ? slot_prim(S, h.slot) : SPT_MISS), h.u, h.v));
-        });
+    __shared__ WarpQueue q[kBlock / 32];
+    RayBatch<STRIDE, false> b{S, rays, nullptr, hits};
+    persistent_trace<kWideStack, false>(q[threadIdx.x >> 5], b, n, next, kWideStack, status);
 }
 
-// The same kernel over a batch in coherence order (ray_order.cu): the k-th ray it takes is order[k],
-// for k below *count (the rays that meet the root box), and its hit goes to place k of hits_ordered,
-// so that neighbouring lanes write neighbouring hits (scattered 16-byte stores cost partial-sector
-// writes in DRAM).
+// The same kernel over a batch in coherence order, for its first *count rays (those that meet the root
+// box).
 template <int STRIDE>
-__global__ void __launch_bounds__(kBlock, 10) k_intersect_df_ordered(DevScene S, const float* __restrict__ rays,
+__global__ void __launch_bounds__(kBlock, 8) k_intersect_df_ordered(const __grid_constant__ DevScene S,
+                                                                 const float* __restrict__ rays,
                                                                  const uint32_t* __restrict__ order,
                                                                  const uint32_t* __restrict__ count,
                                                                  spt_hit* __restrict__ hits_ordered, uint32_t* status,
                                                                  unsigned long long* next) {
-    const uint64_t traced = __ldg(count);
-    persistent_trace(
-        S, traced, next, status, [&](uint64_t k, V3& o, V3& d) { load_ray<STRIDE, true>(rays, __ldg(order + k), o, d); },
-        [&](uint64_t k, const Hit1& h) {
-            __stcs(reinterpret_cast<float4*>(hits_ordered + k),
-                   make_float4(h.t, __uint_as_float(h.found ? slot_prim(S, h.slot) : SPT_MISS), h.u, h.v));
-        });
+    __shared__ WarpQueue q[kBlock / 32];
+    RayBatch<STRIDE, true> b{S, rays, order, hits_ordered};
+    persistent_trace<kWideStack, false>(q[threadIdx.x >> 5], b, __ldg(count), next, kWideStack, status);
 }
 
 // The same kernel with its own work counted (node visits, primitive tests): the work behind the
 // throughput of k_intersect_df, for comparison with the reference traversal's test counts.
-__global__ void __launch_bounds__(kBlock, 10) k_intersect_df_counted(DevScene S, const float* __restrict__ rays,
-                                                                 uint64_t n, spt_hit* __restrict__ hits,
-                                                                 uint32_t* status, unsigned long long* next,
+__global__ void __launch_bounds__(kBlock, 8) k_intersect_df_counted(const __grid_constant__ DevScene S,
+                                                                 const float* __restrict__ rays, uint32_t n,
+                                                                 spt_hit* __restrict__ hits, uint32_t* status,
+                                                                 unsigned long long* next,
                                                                  unsigned long long* counts) {
-    persistent_trace<true>(
-        S, n, next, status, [&](uint64_t i, V3& o, V3& d) { load_ray<8, true>(rays, i, o, d); },
-        [&](uint64_t i, const Hit1& h) {
-            __stcs(reinterpret_cast<float4*>(hits + i),
-                   make_float4(h.t, __uint_as_float(h.found ? slot_prim(S, h.slot) : SPT_MISS), h.u, h.v));
-        },
-        counts);
+    __shared__ WarpQueue q[kBlock / 32];
+    RayBatch<8, false> b{S, rays, nullptr, hits};
+    persistent_trace<kWideStack, true>(q[threadIdx.x >> 5], b, n, next, kWideStack, status, counts);
 }
 
 template <int TRAV, int STRIDE>
@@ -242,7 +254,8 @@ spt_status launch_df(spt_context* ctx, const spt_scene* sc, const float* d_rays,
         k_intersect_df_ordered<STRIDE>
             <<<df_grid<STRIDE>(ctx), kBlock, 0, s>>>(sc->dev, d_rays, order, count, d_hits, ctx->d_status, next);
     else
-        k_intersect_df<STRIDE><<<df_grid<STRIDE>(ctx), kBlock, 0, s>>>(sc->dev, d_rays, n, d_hits, ctx->d_status, next);
+        k_intersect_df<STRIDE><<<df_grid<STRIDE>(ctx), kBlock, 0, s>>>(sc->dev, d_rays, static_cast<uint32_t>(n), d_hits,
+                                                                     ctx->d_status, next);
     SPT_CUDA(ctx, cudaGetLastError());
     return SPT_OK;
 }
@@ -272,7 +285,14 @@ spt_status launch_intersect_t(spt_context* ctx, const spt_scene* sc, const float
             }
             // every per-stream buffer belongs to another stream: the batch's own order
         }
-        return launch_df<STRIDE>(ctx, sc, d_rays, n, d_hits, next, s);
+        // the kernel counts rays in 32 bits: a larger batch goes in runs, each with its own counter
+        constexpr uint64_t kRun = 1ull << 31;
+        for (uint64_t at = 0; at < n; at += kRun) {
+            if (at && (st = fetch_counter(ctx, s, &next)) != SPT_OK) return st;
+            if ((st = launch_df<STRIDE>(ctx, sc, d_rays + STRIDE * at, std::min(kRun, n - at), d_hits + at, next, s)) != SPT_OK)
+                return st;
+        }
+        return SPT_OK;
     } else if (sc->dev.traversal == 1) {
         k_intersect<1, STRIDE><<<blocks_for(n, kBlock), kBlock, 0, s>>>(sc->dev, d_rays, n, d_hits, ctx->d_status);
     } else {
@@ -310,7 +330,13 @@ spt_status launch_intersect_counted(spt_context* ctx, const spt_scene* sc, const
     spt_status st = fetch_counter(ctx, s, &next);
     if (st != SPT_OK) return st;
     static_assert(sizeof(unsigned long long) == 8, "");
-    k_intersect_df_counted<<<df_grid<8>(ctx), kBlock, 0, s>>>(sc->dev, d_rays, n, d_hits, ctx->d_status, next, counts);
+    constexpr uint64_t kRun = 1ull << 31;   // rays the kernel counts in one launch
+    for (uint64_t at = 0; at < n; at += kRun) {
+        if (at && (st = fetch_counter(ctx, s, &next)) != SPT_OK) return st;
+        k_intersect_df_counted<<<df_grid<8>(ctx), kBlock, 0, s>>>(sc->dev, d_rays + 8 * at,
+                                                                static_cast<uint32_t>(std::min(kRun, n - at)), d_hits + at,
+                                                                ctx->d_status, next, counts);
+    }
     SPT_CUDA(ctx, cudaGetLastError());
     return SPT_OK;
 }

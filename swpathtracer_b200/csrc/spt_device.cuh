@@ -54,7 +54,7 @@ struct DevScene {
     const DevMaterial* mat;
     const int* layer_ids;
     const uint4* wnode;         // 8-wide quantized nodes, 5 x uint4 each (wide_build.h)
-    const float4* wtri;         // 3 float4 per triangle in wide-node order: {v0, rank}{e1, type}{e2, leaf}
+    const float4* wtri;         // 3 float4 per primitive in wide-node order: {v0, rank}{e1, prim}{e2, leaf | sphere << 31}
     float root_min[3], root_max[3];
     float bg[3];
     uint32_t n_prims, n_inner, n_leaves, n_nodes2, n_wnodes;

@@ -24,31 +24,31 @@ __device__ __forceinline__ uint32_t byte_of(uint32_t lo, uint32_t hi, int j) {
 
 __device__ __forceinline__ float exp2i(int e) { return __int_as_float((e + 127) << 23); }
 
-struct WideRay {
-    V3 o;
-    float ix, iy, iz;   // 1/d with zero components replaced by a tiny signed value
-    uint32_t inv_oct;   // slot order key: slot ^ inv_oct, ascending = near to far
-};
+// A ray's 1/d has its zero components replaced by a tiny signed value, and inv_oct is its slot order
+// key: slot ^ inv_oct, ascending = near to far.
 
 __device__ __forceinline__ float safe_inv(float d) {
     return 1.0f / (fabsf(d) > 1e-20f ? d : copysignf(1e-20f, d));
 }
 
-__device__ __forceinline__ void wide_node_hits(const DevScene& S, const WideRay& r, uint32_t idx, float best_t,
-                                               uint32_t& g_base, uint32_t& g_hits, uint32_t& g_imask,
-                                               uint32_t& t_base, uint32_t& t_mask) {
-    const uint4* n = S.wnode + 5 * idx;
+// The children of node idx that the ray (o, 1/d) meets before best_t: inner children as near-to-far
+// bits in `hits` (with the node's inner mask and first child), triangles as bits of t_mask from t_base.
+__device__ __forceinline__ void wide_node_hits(const uint4* wnode, V3 o, float ix, float iy, float iz,
+                                               uint32_t inv_oct, uint32_t idx, float best_t, uint32_t& g_base,
+                                               uint32_t& g_hits, uint32_t& g_imask, uint32_t& t_base,
+                                               uint32_t& t_mask) {
+    const uint4* n = wnode + 5ull * idx;
     const uint4 w0 = __ldg(n), w1 = __ldg(n + 1), w2 = __ldg(n + 2), w3 = __ldg(n + 3), w4 = __ldg(n + 4);
     const int ex = static_cast<int8_t>(w0.w & 0xFFu), ey = static_cast<int8_t>((w0.w >> 8) & 0xFFu),
               ez = static_cast<int8_t>((w0.w >> 16) & 0xFFu);
     const uint32_t imask = w0.w >> 24;
-    const float sx = exp2i(ex) * r.ix, sy = exp2i(ey) * r.iy, sz = exp2i(ez) * r.iz;
-    const float ox = (__uint_as_float(w0.x) - r.o.x) * r.ix;
-    const float oy = (__uint_as_float(w0.y) - r.o.y) * r.iy;
-    const float oz = (__uint_as_float(w0.z) - r.o.z) * r.iz;
+    const float sx = exp2i(ex) * ix, sy = exp2i(ey) * iy, sz = exp2i(ez) * iz;
+    const float ox = (__uint_as_float(w0.x) - o.x) * ix;
+    const float oy = (__uint_as_float(w0.y) - o.y) * iy;
+    const float oz = (__uint_as_float(w0.z) - o.z) * iz;
     // The near plane is the low plane when 1/d >= 0.  The choice is made once per node on whole
     // words (four children's planes each), not per child and plane: 12 selects instead of 48.
-    const bool nx = r.ix >= 0.0f, ny = r.iy >= 0.0f, nz = r.iz >= 0.0f;
+    const bool nx = ix >= 0.0f, ny = iy >= 0.0f, nz = iz >= 0.0f;
     const uint32_t nx0 = nx ? w2.x : w3.z, nx1 = nx ? w2.y : w3.w, fx0 = nx ? w3.z : w2.x, fx1 = nx ? w3.w : w2.y;
     const uint32_t ny0 = ny ? w2.z : w4.x, ny1 = ny ? w2.w : w4.y, fy0 = ny ? w4.x : w2.z, fy1 = ny ? w4.y : w2.w;
     const uint32_t nz0 = nz ? w3.x : w4.z, nz1 = nz ? w3.y : w4.w, fz0 = nz ? w4.z : w3.x, fz1 = nz ? w4.w : w3.y;
@@ -65,9 +65,8 @@ __device__ __forceinline__ void wide_node_hits(const DevScene& S, const WideRay&
         const float tfz = __fmaf_rn(static_cast<float>(byte_of(fz0, fz1, j)), sz, oz);
         const float tmin = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, 0.0f));
         const float tmax = fminf(fminf(tfx, tfy), fminf(tfz, best_t));
-        const bool hit = (inner || meta != 0u) && tmin <= tmax;
-        if (hit) {
-            if (inner) hits |= 1u << (j ^ r.inv_oct);
+        if (tmin <= tmax) {   // an empty slot has meta 0: no triangle bits
+            if (inner) hits |= 1u << (j ^ inv_oct);
             else tm |= (meta >> 5) << (meta & 31u);
         }
     }
@@ -89,11 +88,11 @@ __device__ __forceinline__ void wide_candidate(const DevScene& S, uint32_t wslot
     const float4 c = __ldg(S.wtri + 3 * wslot + 2);
     const uint32_t rank = __float_as_uint(a.w);
     float t, u = 0.0f, v = 0.0f;
-    const bool sphere = __float_as_int(b.w) == SPT_PRIM_SPHERE;
+    const bool sphere = (__float_as_uint(c.w) >> 31) != 0u;
     const bool ok = sphere ? sphere_test(f3v(a), c.x, o, d, t) : tri_test(f3v(a), f3v(b), f3v(c), o, d, t, u, v);
     if (!ok || !(t > 0.0f)) return;
     if (!(t < h.t || (h.found && t == h.t && rank < h.slot))) return;
-    const uint32_t leaf = __float_as_uint(c.w);
+    const uint32_t leaf = __float_as_uint(c.w) & 0x7FFFFFFFu;
     if (exact && !inside(S.leaf_box + 6 * leaf, hit_pos(sphere, o, d, t))) return;
     h.t = t;
     h.u = u;
@@ -128,16 +127,12 @@ __device__ __forceinline__ Hit1 closest_hit_wide_pass(const DevScene& S, V3 o, V
                   t1))
             return h;
     }
-    WideRay r;
-    r.o = o;
-    r.ix = safe_inv(d.x);
-    r.iy = safe_inv(d.y);
-    r.iz = safe_inv(d.z);
-    r.inv_oct = (r.ix >= 0.0f ? 0u : 1u) | (r.iy >= 0.0f ? 0u : 2u) | (r.iz >= 0.0f ? 0u : 4u);
+    const float ix = safe_inv(d.x), iy = safe_inv(d.y), iz = safe_inv(d.z);
+    const uint32_t inv_oct = (ix >= 0.0f ? 0u : 1u) | (iy >= 0.0f ? 0u : 2u) | (iz >= 0.0f ? 0u : 4u);
     uint2 stack[kWideStack];
     int sp = 0;
     uint32_t g_base, g_hits, g_imask, t_base, t_mask;
-    wide_node_hits(S, r, 0, h.t, g_base, g_hits, g_imask, t_base, t_mask);
+    wide_node_hits(S.wnode, o, ix, iy, iz, inv_oct, 0, h.t, g_base, g_hits, g_imask, t_base, t_mask);
     for (;;) {
         while (t_mask) {
             const int k = __ffs(t_mask) - 1;
@@ -153,7 +148,7 @@ __device__ __forceinline__ Hit1 closest_hit_wide_pass(const DevScene& S, V3 o, V
         }
         const uint32_t key = __ffs(g_hits) - 1;
         g_hits &= g_hits - 1;
-        const uint32_t s = key ^ r.inv_oct;
+        const uint32_t s = key ^ inv_oct;
         const uint32_t child = g_base + __popc(g_imask & ((1u << s) - 1u));
         if (g_hits) {
             if (sp < kWideStack) {
@@ -163,7 +158,7 @@ __device__ __forceinline__ Hit1 closest_hit_wide_pass(const DevScene& S, V3 o, V
                 atomicOr(overflow, 1u);
             }
         }
-        wide_node_hits(S, r, child, h.t, g_base, g_hits, g_imask, t_base, t_mask);
+        wide_node_hits(S.wnode, o, ix, iy, iz, inv_oct, child, h.t, g_base, g_hits, g_imask, t_base, t_mask);
     }
     return h;
 }
@@ -174,208 +169,296 @@ __device__ __forceinline__ Hit1 closest_hit_wide(const DevScene& S, V3 o, V3 d, 
     return h;
 }
 
-// The same traversal as a resumable state, one node (and its triangles) per step, for kernels that
-// keep a warp's lanes busy by giving a lane a new ray as soon as its ray is finished.
-// A pop reads its 8-byte entry once (not its two halves in several loads): with that, the 48-register
-// closest-hit kernel spills 16 bytes instead of 60 and runs 2,929 instead of 2,718 Mrays/s.
-// REG_TOP keeps the most recent stack entry in registers, so a push followed by its pop touches no
-// local memory.  The path tracer's extend kernel (no register bound) gains 2-5 % from it; the
-// closest-hit kernel, held to 48 registers, would spill more and lose 9 %, so it keeps the plain
-// stack.
-// DEPTH is the compiled stack depth (entries per lane).  A traversal needs at most one entry per wide
-// level below the root for the remaining children of an ancestor plus one per level for postponed
-// triangles, 2 (H - 1) for a wide tree of H levels; wide_stack_bound() gives that bound per scene.
-// step()'s `limit` (1 <= limit <= DEPTH) can hold a traversal to fewer entries; one that needs more
-// sets the overflow status bit instead of writing past the limit.
-// COUNT adds the lane's own work counters (node visits, primitive tests) over all of its rays.
-template <bool REG_TOP, int DEPTH = kWideStack, bool COUNT = false>
-struct WideTraversalT {
+// ---- the same traversal by a warp for 32 rays at a time ----------------------------------------
+//
+// Each lane walks its own ray's nodes; the triangles the lanes come across go to a queue in shared
+// memory, and whenever 32 have gathered the whole warp tests them, one triangle per lane, whichever
+// lanes' rays they belong to.  What bounds the traversal is the number of instructions a warp issues
+// for its lanes (the nodes and triangles sit in L1 and L2): a triangle test by the lane that met it
+// runs with the few lanes that met one in the same step, a queued one with all 32.
+//
+// Two consequences.  A ray keeps walking while its triangles wait, pruned by a best t that does not
+// know them yet: more node visits, never a different answer, since the answer is the minimum of
+// (t, rank) over every candidate and a stale best t is only ever too large.  And a ray is finished
+// when it has no node left and its last queued triangle has been tested.
+//
+// On 2^24 incoherent rays against 1.31M triangles: 3.79 ms a call (order and gather included) against
+// 5.14 with each lane testing its own triangles; 300,007 rays 256 against 372 us; path tracing the
+// layered scene 19.2 against 26.9 ms a render.
+//
+// The per-lane node stack is an array of its own, not a member of the lane's state: a dynamically
+// indexed member keeps the whole struct around it in local memory (the kernels that had it so read
+// and wrote about eleven local words per node visit, more than their node and triangle loads).
+//
+// The lane's best hit sits in shared memory, where the lane that tested the triangle writes it: the
+// 64-bit key t << 32 | rank (t > 0, so its bits order as t does) takes the minimum atomically, and the
+// lane whose key stands writes the barycentrics, the primitive and the leaf.
+constexpr uint32_t kQueue = 64;   // entries: at most 31 left over plus 32 appended before a test
+struct WarpQueue {
+    unsigned long long entry[kQueue];   // triangle record's address | owner lane << 59
+    unsigned long long key[32];
+    float2 uv[32];
+    uint2 id[32];                       // primitive, leaf
+};
+// A warp stops waiting for 32 triangles once this many lanes have nothing else to do.
+constexpr int kWait = 8;
+constexpr unsigned long long kNoHitKey = 0x7F800000FFFFFFFFull;   // t = +inf, any rank
+
+// What the traversal reads of a scene: pointers that stay in the constant bank for a kernel of one
+// scene, or in registers where every lane may have its own.
+struct WideScene {
+    const uint4* wnode;
+    const float4* wtri;
+    const float* leaf_box;
+};
+__device__ __forceinline__ WideScene wide_scene(const DevScene& S) { return WideScene{S.wnode, S.wtri, S.leaf_box}; }
+
+// One lane's ray, without its node stack.  COUNT adds the lane's work (node visits, primitive tests).
+template <int DEPTH, bool COUNT = false>
+struct LaneTrace {
     static_assert(DEPTH >= 1 && DEPTH <= kWideStack, "stack depth out of range");
     V3 o, d;
-    WideRay r;
-    Hit1 h;
-    uint2 stack[DEPTH];
+    float ix, iy, iz;
+    uint32_t inv_oct;
+    float best_t;
+    uint32_t g_base, g_bits;   // pending children of one node: first child, hits (near first) | inner mask << 8
     int sp;
-    uint2 top;
-    bool has_top;
-    uint32_t g_base, g_hits, g_imask, t_base, t_mask;
-    bool exact;
-    uint32_t n_nodes = 0, n_prims = 0;   // COUNT only
+    uint32_t last;             // one past the queue position of the ray's newest triangle
+    bool has, exact;
+    uint32_t n_nodes, n_prims;
 
-    // entries in use: the local ones plus the register top
-    __device__ __forceinline__ bool can_push(int limit) const {
-        return sp + ((REG_TOP && has_top) ? 1 : 0) < limit && sp < DEPTH;
+    __device__ __forceinline__ void clear() {
+        has = exact = false;
+        g_base = g_bits = 0;
+        sp = 0;
+        last = 0;
+        best_t = inf_f();
+        o = d = v3(0.0f, 0.0f, 0.0f);
+        ix = iy = iz = 0.0f;
+        inv_oct = 0;
+        n_nodes = n_prims = 0;
     }
-    __device__ __forceinline__ void push(uint2 e) {
-        if (!REG_TOP) {
-            stack[sp++] = e;
-            return;
-        }
-        if (has_top) stack[sp++] = top;
-        top = e;
-        has_top = true;
-    }
-    // With REG_TOP the register entry is the stack's top whenever the stack is not empty: a pop
-    // returns it and at once loads the next entry from local memory into the register, so that load
-    // has the whole next node visit to arrive before the following pop needs it.
-    __device__ __forceinline__ bool empty() const { return REG_TOP ? !has_top : sp == 0; }
-    __device__ __forceinline__ uint2 pop() {
-        if (!REG_TOP) return stack[--sp];
-        const uint2 r = top;
-        if (sp > 0) top = stack[--sp];
-        else has_top = false;
-        return r;
+    __device__ __forceinline__ bool walking() const { return (g_bits & 0xFFu) != 0u || sp > 0; }
+
+    // From the first node again, with the lane's o and d (in exact mode after a failed inside test).
+    __device__ __forceinline__ void restart(WarpQueue& Q, uint32_t qhead, bool exact_) {
+        exact = exact_;
+        best_t = inf_f();
+        sp = 0;
+        last = qhead;
+        g_base = 0;                          // a pending visit of node 0: one hit child (slot 0, whose
+        g_bits = (1u << inv_oct) | (1u << 8);   // near-to-far key is inv_oct) of a parent of node 0
+        Q.key[threadIdx.x & 31u] = kNoHitKey;
     }
 
-    // Returns false when the ray is already finished (empty scene or root box missed).  The root node
-    // itself is visited by the first step(): a lane that takes a new ray while the rest of its warp
-    // is mid-traversal then tests the root's children together with the other lanes' node visits,
-    // not alone in the refill branch.
-    __device__ __forceinline__ bool start(const DevScene& S, V3 o_, V3 d_, bool exact_ = false) {
+    // Takes a ray; false when the scene's root box (the reference's own slab test) is missed.  The root
+    // node is visited by the next step, together with the other lanes' node visits.
+    __device__ __forceinline__ bool start(const float* root_min, const float* root_max, V3 o_, V3 d_, WarpQueue& Q,
+                                          uint32_t qhead) {
         o = o_;
         d = d_;
-        exact = exact_;
-        h.t = inf_f();
-        h.u = h.v = 0.0f;
-        h.slot = 0;
-        h.leaf = 0;
-        h.found = false;
-        sp = 0;
-        has_top = false;
-        if (S.empty) return false;
         const RayInv ri = ray_inv(o, d);
         float t0, t1;
-        if (!slab(ri, S.root_min[0], S.root_min[1], S.root_min[2], S.root_max[0], S.root_max[1], S.root_max[2], t0, t1))
-            return false;
-        r.o = o;
+        has = slab(ri, root_min[0], root_min[1], root_min[2], root_max[0], root_max[1], root_max[2], t0, t1);
+        if (!has) return false;
         // safe_inv without dividing again: 1/d is already in ri unless |d| <= 1e-20
-        r.ix = fabsf(d.x) > 1e-20f ? ri.inv.x : copysignf(1.0f / 1e-20f, d.x);
-        r.iy = fabsf(d.y) > 1e-20f ? ri.inv.y : copysignf(1.0f / 1e-20f, d.y);
-        r.iz = fabsf(d.z) > 1e-20f ? ri.inv.z : copysignf(1.0f / 1e-20f, d.z);
-        r.inv_oct = (r.ix >= 0.0f ? 0u : 1u) | (r.iy >= 0.0f ? 0u : 2u) | (r.iz >= 0.0f ? 0u : 4u);
-        // a pending visit of node 0: one hit child (slot 0, whose near-to-far key is inv_oct) of a
-        // parent whose first child is node 0
-        g_base = 0;
-        g_imask = 1u;
-        g_hits = 1u << r.inv_oct;
-        t_base = 0;
-        t_mask = 0;
+        ix = fabsf(d.x) > 1e-20f ? ri.inv.x : copysignf(1.0f / 1e-20f, d.x);
+        iy = fabsf(d.y) > 1e-20f ? ri.inv.y : copysignf(1.0f / 1e-20f, d.y);
+        iz = fabsf(d.z) > 1e-20f ? ri.inv.z : copysignf(1.0f / 1e-20f, d.z);
+        inv_oct = (ix >= 0.0f ? 0u : 1u) | (iy >= 0.0f ? 0u : 2u) | (iz >= 0.0f ? 0u : 4u);
+        restart(Q, qhead, false);
         return true;
     }
 
-    // One step: the pending triangles, then the next node.  Returns false once the ray is done.
-    // When fewer than 1/8 of the warp's active lanes have triangles to test and this lane still has
-    // nodes to visit, its triangles wait on the stack (tag bit 31 of .x) so the warp keeps traversing
-    // together (after the triangle postponing of Ylitie et al., HPG 2017).  Measured on 2^24
-    // incoherent rays: 2,103 -> 2,568 Mrays/s.  The order of the candidates does not change the
-    // result, which is the minimum over (t, rank).  A popped triangle entry is tested at the next step
-    // (no node work in hand), so every entry is postponed at most once.
-    __device__ __forceinline__ bool step(const DevScene& S, uint32_t* overflow, int limit = DEPTH) {
-        const unsigned act = __activemask();
-        const unsigned tri = __ballot_sync(act, t_mask != 0u);
-        if (t_mask && g_hits && can_push(limit) && 8 * __popc(tri) < __popc(act)) {
-            push(make_uint2(t_base | 0x80000000u, t_mask));
-            t_mask = 0;
-        }
-        while (t_mask) {
-            const int k = __ffs(t_mask) - 1;
-            t_mask &= t_mask - 1;
-            wide_candidate(S, t_base + k, o, d, h, exact);
-            if (COUNT) ++n_prims;
-        }
-        if (!g_hits) {
-            if (empty()) return false;
-            const uint2 e = pop();
-            if (e.x & 0x80000000u) {   // postponed triangles
-                t_base = e.x & 0x7FFFFFFFu;
-                t_mask = e.y;
-                return true;
-            }
+    // The lane's next node; its triangles come back as a run (t_base, t_mask).  A traversal that needs
+    // more than `limit` stack entries sets the overflow status bit instead of pushing.
+    __device__ __forceinline__ void visit(const uint4* wnode, uint2 (&stack)[DEPTH], int limit, uint32_t* status,
+                                          uint32_t& t_base, uint32_t& t_mask) {
+        if (!(g_bits & 0xFFu)) {
+            const uint2 e = stack[--sp];   // one 8-byte load
             g_base = e.x;
-            g_hits = e.y & 0xFFu;
-            g_imask = e.y >> 8;
+            g_bits = e.y;
         }
-        const uint32_t key = __ffs(g_hits) - 1;
-        g_hits &= g_hits - 1;
-        const uint32_t s = key ^ r.inv_oct;
-        const uint32_t child = g_base + __popc(g_imask & ((1u << s) - 1u));
-        if (g_hits) {
-            if (can_push(limit)) push(make_uint2(g_base, g_hits | (g_imask << 8)));
-            else atomicOr(overflow, 1u);
+        const uint32_t s = static_cast<uint32_t>(__ffs(g_bits) - 1) ^ inv_oct;
+        g_bits &= g_bits - 1;
+        const uint32_t child = g_base + __popc((g_bits >> 8) & ((1u << s) - 1u));
+        if (g_bits & 0xFFu) {
+            if (sp < limit) stack[sp++] = make_uint2(g_base, g_bits);
+            else atomicOr(status, 1u);
         }
-        wide_node_hits(S, r, child, h.t, g_base, g_hits, g_imask, t_base, t_mask);
+        uint32_t hits, imask;
+        wide_node_hits(wnode, o, ix, iy, iz, inv_oct, child, best_t, g_base, hits, imask, t_base, t_mask);
+        g_bits = hits | (imask << 8);
         if (COUNT) ++n_nodes;
-        return true;
-    }
-
-    // After step() returned false: true if the result is final; false if the final hit failed the
-    // deferred inside test and the traversal restarted in exact mode (keep stepping).
-    __device__ __forceinline__ bool finish(const DevScene& S) {
-        if (exact || final_inside(S, h, o, d)) return true;
-        start(S, o, d, true);
-        return false;
     }
 };
 
+// Tests the oldest nq <= 32 triangles of the queue, one per lane, by the whole warp.
+template <int DEPTH, bool COUNT>
+__device__ __forceinline__ void test_queued(WarpQueue& Q, uint32_t& qhead, uint32_t nq, const WideScene& W,
+                                            LaneTrace<DEPTH, COUNT>& tr, unsigned exact_lanes) {
+    const uint32_t lane = threadIdx.x & 31u;
+    __syncwarp();   // the entries are written
+    const bool mine = lane < nq;
+    const unsigned long long e = Q.entry[(qhead + lane) & (kQueue - 1)];
+    const uint32_t owner = mine ? static_cast<uint32_t>(e >> 59) : lane;
+    const V3 o = v3(__shfl_sync(0xFFFFFFFFu, tr.o.x, owner), __shfl_sync(0xFFFFFFFFu, tr.o.y, owner),
+                    __shfl_sync(0xFFFFFFFFu, tr.o.z, owner));
+    const V3 d = v3(__shfl_sync(0xFFFFFFFFu, tr.d.x, owner), __shfl_sync(0xFFFFFFFFu, tr.d.y, owner),
+                    __shfl_sync(0xFFFFFFFFu, tr.d.z, owner));
+    const float* box = W.leaf_box;
+    if (exact_lanes)   // rare: the owner's scene for the inside test
+        box = reinterpret_cast<const float*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(box), owner));
+    qhead += nq;
+    bool ok = false;
+    float t = 0.0f, u = 0.0f, v = 0.0f;
+    uint32_t prim = 0, leaf = 0;
+    unsigned long long key = 0;
+    if (mine) {
+        const float4* p = reinterpret_cast<const float4*>(e & ((1ull << 59) - 1));
+        const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+        prim = __float_as_uint(b.w);
+        leaf = __float_as_uint(c.w) & 0x7FFFFFFFu;
+        const bool sphere = (__float_as_uint(c.w) >> 31) != 0u;
+        ok = sphere ? sphere_test(f3v(a), c.x, o, d, t) : tri_test(f3v(a), f3v(b), f3v(c), o, d, t, u, v);
+        key = (static_cast<unsigned long long>(__float_as_uint(t)) << 32) | __float_as_uint(a.w);
+        ok = ok && t > 0.0f && t < inf_f() && key < Q.key[owner];
+        if (ok && ((exact_lanes >> owner) & 1u)) ok = inside(box + 6ull * leaf, hit_pos(sphere, o, d, t));
+        if (COUNT) ++tr.n_prims;
+    }
+    __syncwarp();   // entries and keys are read
+    if (__any_sync(0xFFFFFFFFu, ok)) {
+        if (ok) atomicMin(&Q.key[owner], key);
+        __syncwarp();
+        if (ok && Q.key[owner] == key) {   // ranks are unique, so one lane per owner
+            Q.uv[owner] = make_float2(u, v);
+            Q.id[owner] = make_uint2(prim, leaf);
+        }
+        __syncwarp();
+        tr.best_t = __uint_as_float(static_cast<uint32_t>(Q.key[lane] >> 32));
+    }
+}
+
+// One step of the warp: every walking lane visits a node, and the triangles found are queued and
+// tested 32 at a time (fewer when too many lanes wait for theirs).
+template <int DEPTH, bool COUNT>
+__device__ __forceinline__ void warp_step(WarpQueue& Q, uint32_t& qhead, uint32_t& qtail, const WideScene& W,
+                                          LaneTrace<DEPTH, COUNT>& tr, uint2 (&stack)[DEPTH], int limit,
+                                          uint32_t* status, unsigned exact_lanes) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const unsigned lt = (1u << lane) - 1u;
+    uint32_t t_base = 0, t_mask = 0;
+    if (tr.walking()) tr.visit(W.wnode, stack, limit, status, t_base, t_mask);
+    const unsigned long long first =
+        reinterpret_cast<unsigned long long>(W.wtri + 3ull * t_base) | (static_cast<unsigned long long>(lane) << 59);
+    unsigned found;
+    do {
+        found = __ballot_sync(0xFFFFFFFFu, t_mask != 0u);
+        if (t_mask) {
+            const uint32_t k = __ffs(t_mask) - 1;
+            t_mask &= t_mask - 1;
+            const uint32_t pos = qtail + __popc(found & lt);
+            Q.entry[pos & (kQueue - 1)] = first + k * (3u * sizeof(float4));
+            tr.last = pos + 1;
+        }
+        qtail += __popc(found);
+        const uint32_t n = qtail - qhead;
+        bool go = n >= 32;
+        if (!found && n) {
+            const bool walks = tr.walking();
+            const unsigned waits = __ballot_sync(0xFFFFFFFFu, tr.has && !walks && static_cast<int>(qhead - tr.last) < 0);
+            go = __popc(waits) >= kWait || !__any_sync(0xFFFFFFFFu, walks);
+        }
+        if (go) test_queued(Q, qhead, n < 32 ? n : 32u, W, tr, exact_lanes);
+    } while (found);
+}
+
 // Persistent warps with dynamic ray fetch (after Aila & Laine, "Understanding the Efficiency of Ray
 // Traversal on GPUs", HPG 2009): a lane whose ray is finished takes the next ray at once instead of
-// idling until the warp's longest ray ends.  Ray indices come from a warp-local pool refilled
-// kChunk at a time from one global counter, so the counter sees one atomic per kChunk rays.  32 is
-// the least that works (one refill may hand up to 32 lanes rays from a fresh chunk): against 64 it
-// measured +0.6 % on the ordered incoherent queries and +4.6 % / +8.2 % on the box and layered path
-// tracing (a shorter tail, and the ordered neighbours stay together); 128 lost 3 %.
-// load(i, o, d) fetches ray i; store(i, h) writes its result.
+// idling until the warp's longest ray ends.  Ray indices come from a warp-local pool refilled `chunk`
+// at a time from one global counter, so the counter sees one atomic per chunk.  32 rays per chunk:
+// against 64 it measured +0.6 % on the ordered incoherent queries and +4.6 % / +8.2 % on the box and
+// layered path tracing (a shorter tail, and the ordered neighbours stay together); 128 lost 3 %.
 constexpr uint32_t kChunk = 32;
-static_assert(kChunk >= 32, "a refill takes up to 32 rays from one fresh chunk");
-// Refill once this many lanes wait for a ray (or no lane is busy): the refill branch runs with only
-// the waiting lanes, so batching it pays a little (2,674 -> 2,690 Mrays/s at 4; 2 and 8 gain less).
+// Lanes are served (hit stored, next ray taken) once this many wait, or no lane is busy.
 constexpr int kRefill = 4;
 
-// COUNT: adds the kernel's own node visits and primitive tests to counts[0] / counts[1].
-template <bool COUNT = false, typename Load, typename Store>
-__device__ __forceinline__ void persistent_trace(const DevScene& S, uint64_t n, unsigned long long* next,
-                                                 uint32_t* overflow, Load load, Store store,
-                                                 unsigned long long* counts = nullptr) {
-    const uint32_t lane = threadIdx.x & 31;
+// source: load(i, o, d) fetches ray i (and, for a kernel of many scenes, the lane's scene), root_min()
+// and root_max() are its scene's root box, scene() its WideScene, store(i, t, prim, u, v) takes the hit.
+template <int DEPTH, bool COUNT, typename Source>
+__device__ __forceinline__ void persistent_trace(WarpQueue& Q, Source& src, uint32_t n, unsigned long long* next,
+                                                 int limit, uint32_t* status, unsigned long long* counts = nullptr) {
+    const uint32_t lane = threadIdx.x & 31u;
     const unsigned lt = (1u << lane) - 1u;
-    WideTraversalT<false, kWideStack, COUNT> tr;
-    bool active = false, exhausted = false;
-    uint64_t mine = 0;
-    unsigned long long pool = 0, pool_end = 0;  // warp-uniform
+    uint2 stack[DEPTH];
+    LaneTrace<DEPTH, COUNT> tr;
+    tr.clear();
+    uint32_t qhead = 0, qtail = 0, mine = 0, pool = 0, pool_end = 0;
+    unsigned exact_lanes = 0;
+    bool exhausted = false;
     for (;;) {
-        const unsigned need = __ballot_sync(0xFFFFFFFFu, !active && !exhausted);
-        const unsigned busy = __ballot_sync(0xFFFFFFFFu, active);
+        const bool fin = tr.has && !tr.walking() && static_cast<int>(qhead - tr.last) >= 0;
+        const unsigned need = __ballot_sync(0xFFFFFFFFu, fin || (!tr.has && !exhausted));
+        const unsigned busy = __ballot_sync(0xFFFFFFFFu, tr.has && !fin);
         if (need && (__popc(need) >= kRefill || !busy)) {
-            const uint32_t cnt = __popc(need), rank = __popc(need & lt);
-            const unsigned long long have = pool_end - pool;
-            unsigned long long fresh = 0;
-            if (have < cnt) {
-                if (lane == 0) fresh = atomicAdd(next, static_cast<unsigned long long>(kChunk));
-                fresh = __shfl_sync(0xFFFFFFFFu, fresh, 0);
-            }
-            if (!active && !exhausted) {
-                mine = rank < have ? pool + rank : fresh + (rank - have);
-                if (mine >= n) {
-                    exhausted = true;
+            if (fin) {
+                const unsigned long long key = Q.key[lane];
+                if (key == kNoHitKey) {
+                    src.store(mine, inf_f(), SPT_MISS, 0.0f, 0.0f);
+                    tr.has = false;
                 } else {
+                    // the deferred inside test of the final hit (o + d*t is the same float expression
+                    // for both primitive kinds); when it fails the ray is traced again, with the test
+                    // applied to every candidate
+                    const float t = __uint_as_float(static_cast<uint32_t>(key >> 32));
+                    const uint2 id = Q.id[lane];
+                    if (tr.exact || inside(src.scene().leaf_box + 6ull * id.y, tr.o + tr.d * t)) {
+                        const float2 uv = Q.uv[lane];
+                        src.store(mine, t, id.x, uv.x, uv.y);
+                        tr.has = false;
+                    } else {
+                        tr.restart(Q, qhead, true);
+                    }
+                }
+            }
+            const bool want = !tr.has && !exhausted;
+            const unsigned wants = __ballot_sync(0xFFFFFFFFu, want);
+            const uint32_t cnt = __popc(wants), rank = __popc(wants & lt), have = pool_end - pool;
+            uint32_t fresh = 0, extra = 0;
+            if (have < cnt) {
+                unsigned long long f = 0;
+                if (lane == 0) f = atomicAdd(next, static_cast<unsigned long long>(kChunk));
+                f = __shfl_sync(0xFFFFFFFFu, f, 0);
+                if (f < n) {
+                    fresh = static_cast<uint32_t>(f);
+                    extra = min(kChunk, n - fresh);
+                }
+            }
+            if (want) {
+                if (rank < have) {
+                    mine = pool + rank;
+                } else if (rank - have < extra) {
+                    mine = fresh + (rank - have);
+                } else {
+                    exhausted = true;
+                }
+                if (!exhausted) {
                     V3 o, d;
-                    load(mine, o, d);
-                    active = tr.start(S, o, d);
-                    if (!active) store(mine, tr.h);
+                    src.load(mine, o, d);
+                    if (!tr.start(src.root_min(), src.root_max(), o, d, Q, qhead))
+                        src.store(mine, inf_f(), SPT_MISS, 0.0f, 0.0f);
                 }
             }
             if (have < cnt) {
-                pool = fresh + (cnt - have);
-                pool_end = fresh + kChunk;
+                pool = fresh + min(cnt - have, extra);
+                pool_end = fresh + extra;
             } else {
                 pool += cnt;
             }
+            exact_lanes = __ballot_sync(0xFFFFFFFFu, tr.has && tr.exact);
+            if (__all_sync(0xFFFFFFFFu, !tr.has && exhausted)) break;
         }
-        if (__all_sync(0xFFFFFFFFu, !active && exhausted)) break;
-        if (active && !tr.step(S, overflow) && tr.finish(S)) {
-            store(mine, tr.h);
-            active = false;
-        }
+        warp_step(Q, qhead, qtail, src.scene(), tr, stack, limit, status, exact_lanes);
     }
     if (COUNT) {
         unsigned long long a = tr.n_nodes, b = tr.n_prims;
