@@ -204,11 +204,11 @@ struct PathRays {
 
 // Persistent extend: lanes take live slots from the iteration's counter as their rays finish.
 // DEPTH: the lane's traversal stack depth (tune.stack); W.stack_limit may hold it lower.  MANY: the
-// batch's jobs are of several scenes (S is the one scene otherwise).  Blocks per SM by measurement:
-// the layered scene 19.1 ms at 8 and 19.4 at 7 (72 registers), the box level; the batch, whose lanes
-// hold their scene's pointers, 20.0 ms at 7 and 20.9 at 8.
+// batch's jobs are of several scenes (S is the one scene otherwise).  Seven blocks
+// per SM (72 registers): the layered scene renders in 18.2 ms, 18.4 at eight and 19.0 at six; a batch of
+// eight scenes in 18.9, 19.9 at six.
 template <int DEPTH, bool MANY>
-__global__ void __launch_bounds__(128, MANY ? 7 : 8) k_extend_df(const __grid_constant__ Wave W, const __grid_constant__ DevScene S,
+__global__ void __launch_bounds__(128, 7) k_extend_df(const __grid_constant__ Wave W, const __grid_constant__ DevScene S,
                                                    Counters* __restrict__ ctr, const __grid_constant__ PathBuf cur,
                                                    float4* __restrict__ hits, uint32_t* status) {
     __shared__ WarpQueue q[4];
