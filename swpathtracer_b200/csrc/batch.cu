@@ -121,6 +121,7 @@ spt_status spt_autotune(spt_context* ctx, const spt_batch_job* jobs, uint32_t n_
         *out = best;
         return SPT_OK;
     }
+    best.traversal = 2;   // what the default (-1) runs, by name: the result says which traversal was timed
     SPT_CUDA(ctx, cudaSetDevice(ctx->device));
     // scratch images for the trials
     size_t total_px = 0;
