@@ -59,8 +59,8 @@ struct RayBatch {
 };
 
 // Persistent variant: wide traversal, lanes refilled from a global ray counter (traverse_wide.cuh).
-// 8 blocks of 128 per SM (at most 64 registers): on 2^24 incoherent rays 3.86 ms a step against 4.22 at
-// 10 blocks (48 registers, 150 bytes spilled), 3.93 at 7 and 4.22 at 6.
+// 8 blocks of 128 per SM (at most 64 registers): when the triangle queue came in, 2^24 incoherent rays
+// took 3.86 ms a call at 8 blocks, 4.22 at 10 (48 registers, 150 bytes spilled), 3.93 at 7, 4.22 at 6.
 template <int STRIDE>
 __global__ void __launch_bounds__(kBlock, 8) k_intersect_df(const __grid_constant__ DevScene S,
                                                          const float* __restrict__ rays, uint32_t n,

@@ -242,9 +242,9 @@ __device__ __forceinline__ Hit1 closest_hit_wide(const DevScene& S, V3 o, V3 d, 
 // (t, rank) over every candidate and a stale best t is only ever too large.  And a ray is finished
 // when it has no node left and its last queued triangle has been tested.
 //
-// On 2^24 incoherent rays against 1.31M triangles: 3.79 ms a call (order and gather included) against
-// 5.14 with each lane testing its own triangles; 300,007 rays 256 against 372 us; path tracing the
-// layered scene 19.2 against 26.9 ms a render.
+// On 2^24 incoherent rays against 1.31M triangles the call (order and gather included) takes 3.00 ms, and
+// took 5.14 with each lane testing its own triangles and the lane's state in local memory; 300,007
+// rays 199 against 372 us; path tracing the layered scene 16.6 against 26.9 ms a render.
 //
 // The per-lane node stack is an array of its own, not a member of the lane's state: a dynamically
 // indexed member keeps the whole struct around it in local memory (the kernels that had it so read
@@ -253,12 +253,14 @@ __device__ __forceinline__ Hit1 closest_hit_wide(const DevScene& S, V3 o, V3 d, 
 // The lane's best hit sits in shared memory, where the lane that tested the triangle writes it: the
 // 64-bit key t << 32 | rank (t > 0, so its bits order as t does) takes the minimum atomically, and the
 // lane whose key stands writes the barycentrics, the primitive and the leaf.
-constexpr uint32_t kQueue = 64;   // entries: at most 31 left over plus 32 appended before a test
+constexpr uint32_t kQueue = 128;   // entries, a power of two of at least 64
 struct WarpQueue {
     unsigned long long entry[kQueue];   // triangle record's address | owner lane << 59
     unsigned long long key[32];
     float2 uv[32];
     uint2 id[32];                       // primitive, leaf
+    uint32_t tail;                      // one past the newest entry (the same as the warp's qtail)
+    uint32_t pool, pool_end, first;     // the warp's rays in hand, and the first ray the counter hands out
 };
 // A warp stops waiting for 32 triangles once this many lanes have nothing else to do (4, 8 and 16 measure
 // alike).
@@ -407,31 +409,47 @@ __device__ __forceinline__ void warp_step(WarpQueue& Q, uint32_t& qhead, uint32_
                                           LaneTrace<DEPTH, COUNT>& tr, uint2 (&stack)[DEPTH], int limit,
                                           uint32_t* status, unsigned exact_lanes) {
     const uint32_t lane = threadIdx.x & 31u;
-    const unsigned lt = (1u << lane) - 1u;
     uint32_t t_base = 0, t_mask = 0;
     if (tr.walking()) tr.visit(W.wnode, stack, limit, status, t_base, t_mask);
     const unsigned long long first =
         reinterpret_cast<unsigned long long>(W.wtri + 3ull * t_base) | (static_cast<unsigned long long>(lane) << 59);
+    // Room for all of them (31 at most are left over, and a step finds 15 on average): each lane reserves a
+    // run of places with one shared-memory atomic and fills it.  Otherwise one triangle per lane at a
+    // time, with tests in between.  (Appending one per lane at a time throughout took six rounds of
+    // ballots a step: 3.44 against 3.00 ms a call on 2^24 incoherent rays, the layered path tracing 18.3
+    // against 16.6 ms.)
+    const uint32_t mine = __popc(t_mask), all = __reduce_add_sync(0xFFFFFFFFu, mine);
+    if (all && qtail - qhead + all <= kQueue) {
+        if (mine) {
+            uint32_t pos = atomicAdd(&Q.tail, mine);
+            tr.last = pos + mine;
+            for (; t_mask; t_mask &= t_mask - 1, ++pos)
+                Q.entry[pos & (kQueue - 1)] = first + static_cast<uint32_t>(__ffs(t_mask) - 1) * (3u * sizeof(float4));
+        }
+        qtail += all;
+    }
     unsigned found;
     do {
         found = __ballot_sync(0xFFFFFFFFu, t_mask != 0u);
-        if (t_mask) {
-            const uint32_t k = __ffs(t_mask) - 1;
-            t_mask &= t_mask - 1;
-            const uint32_t pos = qtail + __popc(found & lt);
-            Q.entry[pos & (kQueue - 1)] = first + k * (3u * sizeof(float4));
-            tr.last = pos + 1;
+        if (found) {
+            if (t_mask) {
+                const uint32_t pos = qtail + __popc(found & ((1u << lane) - 1u));
+                Q.entry[pos & (kQueue - 1)] = first + static_cast<uint32_t>(__ffs(t_mask) - 1) * (3u * sizeof(float4));
+                t_mask &= t_mask - 1;
+                tr.last = pos + 1;
+            }
+            qtail += __popc(found);
+            if (lane == 0) Q.tail = qtail;
         }
-        qtail += __popc(found);
         const uint32_t n = qtail - qhead;
         bool go = n >= 32;
-        if (!found && n) {
+        if (!found && n && !go) {
             const bool walks = tr.walking();
             const unsigned waits = __ballot_sync(0xFFFFFFFFu, tr.has && !walks && static_cast<int>(qhead - tr.last) < 0);
             go = __popc(waits) >= kWait || !__any_sync(0xFFFFFFFFu, walks);
         }
-        if (go) test_queued(Q, qhead, n < 32 ? n : 32u, W, tr, exact_lanes);
-    } while (found);
+        if (go) test_queued(Q, qhead, min(n, 32u), W, tr, exact_lanes);
+    } while (found || qtail - qhead >= 32);
 }
 
 // Persistent warps with dynamic ray fetch (after Aila & Laine, "Understanding the Efficiency of Ray
@@ -455,7 +473,18 @@ __device__ __forceinline__ void persistent_trace(WarpQueue& Q, Source& src, uint
     uint2 stack[DEPTH];
     LaneTrace<DEPTH, COUNT> tr;
     tr.clear();
-    uint32_t qhead = 0, qtail = 0, mine = 0, pool = 0, pool_end = 0;
+    uint32_t qhead = 0, qtail = 0, mine = 0;
+    if (lane == 0) {
+        Q.tail = 0;
+        // Small batches spread over the warps, so that a ray's chain of dependent loads has a warp for
+        // itself.  A warp's first chunk goes by its number; the counter hands out those after.
+        const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+        const uint32_t chunk = min(kChunk, max(1u, n / warps));
+        Q.first = warps * chunk;
+        Q.pool = min(n, (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * chunk);
+        Q.pool_end = min(n, Q.pool + chunk);
+    }
+    __syncwarp();
     unsigned exact_lanes = 0;
     bool exhausted = false;
     for (;;) {
@@ -485,12 +514,13 @@ __device__ __forceinline__ void persistent_trace(WarpQueue& Q, Source& src, uint
             }
             const bool want = !tr.has && !exhausted;
             const unsigned wants = __ballot_sync(0xFFFFFFFFu, want);
-            const uint32_t cnt = __popc(wants), rank = __popc(wants & lt), have = pool_end - pool;
+            const uint32_t pool = Q.pool, have = Q.pool_end - pool;
+            const uint32_t cnt = __popc(wants), rank = __popc(wants & lt);
             uint32_t fresh = 0, extra = 0;
             if (have < cnt) {
                 unsigned long long f = 0;
                 if (lane == 0) f = atomicAdd(next, static_cast<unsigned long long>(kChunk));
-                f = __shfl_sync(0xFFFFFFFFu, f, 0);
+                f = __shfl_sync(0xFFFFFFFFu, f, 0) + Q.first;
                 if (f < n) {
                     fresh = static_cast<uint32_t>(f);
                     extra = min(kChunk, n - fresh);
@@ -511,12 +541,12 @@ __device__ __forceinline__ void persistent_trace(WarpQueue& Q, Source& src, uint
                         src.store(mine, inf_f(), SPT_MISS, 0.0f, 0.0f);
                 }
             }
-            if (have < cnt) {
-                pool = fresh + min(cnt - have, extra);
-                pool_end = fresh + extra;
-            } else {
-                pool += cnt;
+            __syncwarp();
+            if (lane == 0) {
+                Q.pool = have < cnt ? fresh + min(cnt - have, extra) : pool + cnt;
+                if (have < cnt) Q.pool_end = fresh + extra;
             }
+            __syncwarp();
             exact_lanes = __ballot_sync(0xFFFFFFFFu, tr.has && tr.exact);
             if (__all_sync(0xFFFFFFFFu, !tr.has && exhausted)) break;
         }
