@@ -1,15 +1,19 @@
 // pathtrace.cu -- the path tracer (integrators/pathtracer.cpp:12-147) as a wavefront over a batch
 // of scenes.
 //
-// A pool of path slots (SoA, ping-pong) is refilled with new camera paths as old ones end.  Each
-// iteration runs four kernels:
+// A pool of path slots (SoA, ping-pong) holds the live paths.  Each iteration runs
 //
-//   k_generate  camera rays for free slots (pixel sampler + camera, pathtracer.cpp:104-113)
+//   k_generate  camera rays for free slots (pixel sampler + camera, pathtracer.cpp:104-113); once, ahead
+//               of the loop, when the pool holds every camera path
 //   k_extend    closest hit for every live slot (traverse*.cuh, the ray casters' traversal)
 //   k_shade     emission, layered BSDF walk, russian roulette and the next ray
 //               (pathtracer.cpp:21-54); surviving paths are appended, warp-aggregated, to the other
-//               buffer; finished paths add their radiance to their scene's image
-//   k_advance   one thread: moves the counters to the next iteration
+//               buffer; finished paths add their radiance to their scene's image; the last block to
+//               finish moves the counters to the next iteration
+//
+// (New paths go behind the live ones, in a kernel of their own: appended by k_shade's lanes in the room of
+// ended paths, they mixed camera rays into the warps of bounced ones, and the layered scene took 17.5
+// instead of 16.3 ms.)
 //
 // A batch is a table of jobs (scene + camera + settings); the camera paths of all jobs form one index
 // space, so scenes of very different sizes share the pool, and the iterations are replayed from one
@@ -57,7 +61,7 @@ struct Counters {
     uint32_t n_alive;               // live slots at the start of the iteration (in the current buffer)
     uint32_t n_next;                // slots appended to the other buffer by k_shade
     uint32_t iterations;
-    uint32_t spare;
+    uint32_t done;                  // blocks of the running k_shade that have finished
     uint32_t rec_count;             // training records written into the current generation
     uint32_t rec_gen;               // generation of the record buffer (bumped when it is consumed)
     uint32_t train_on;              // record training data
@@ -78,14 +82,27 @@ struct GuideIO {
     float4* recx;          // 2 float4 per record: throughput at the record, radiance gathered after it
 };
 
+// What k_shade does at the end of an iteration that ends a pass of the device-side loop.
+struct LoopEnd {
+    uint32_t on, max_iterations;
+    uint32_t* status;
+    cudaGraphConditionalHandle loop;
+};
+
 constexpr uint32_t kNoRec = 0xFFFFFFFFu;
 constexpr uint32_t kRecBatches = 4;   // training records held per render: this many optimiser batches
 constexpr uint32_t kTrainEpochs = 4;  // optimiser passes over each filled record buffer
 
-__device__ __forceinline__ uint32_t n_new_paths(const Wave& W, const Counters& c) {
-    const unsigned long long rem = W.total - c.next_path;
-    const uint32_t room = W.capacity - c.n_alive;
+// New camera paths of this iteration: as many as are left and have room.
+__device__ __forceinline__ uint32_t n_new_paths(const Wave& W, uint32_t n_alive, unsigned long long next_path) {
+    const unsigned long long rem = W.total - next_path;
+    const uint32_t room = W.capacity - n_alive;
     return rem < room ? static_cast<uint32_t>(rem) : room;
+}
+// Slots of this iteration: the live paths, then the new ones.
+__device__ __forceinline__ uint32_t n_slots(const Wave& W, const Counters* ctr) {
+    const uint32_t n_alive = ctr->n_alive;
+    return n_alive + n_new_paths(W, n_alive, ctr->next_path);
 }
 
 __device__ __forceinline__ uint32_t job_of(const Wave& W, unsigned long long g) {
@@ -98,48 +115,53 @@ __device__ __forceinline__ uint32_t job_of(const Wave& W, unsigned long long g) 
     return lo;
 }
 
-__global__ void __launch_bounds__(256) k_generate(Wave W, const Counters* __restrict__ ctr, PathBuf cur) {
-    const Counters c = *ctr;
-    const uint32_t n_new = n_new_paths(W, c);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_new; i += gridDim.x * blockDim.x) {
-        const unsigned long long g = c.next_path + i;
-        const uint32_t j = job_of(W, g);
-        const PtJob& J = W.jobs[j];
-        const unsigned long long lg = g - J.first;
-        const uint32_t sr = static_cast<uint32_t>(lg / J.npix);
-        const uint32_t pix = static_cast<uint32_t>(lg - static_cast<unsigned long long>(sr) * J.npix);
-        const uint32_t si = J.s_begin + sr;   // sample index within the pixel's spp
-        const uint32_t xx = pix % J.cam.vp_width, yy = pix / J.cam.vp_width;
-        const uint32_t x = J.cam.vp_left + xx, y = J.cam.vp_top + yy;
-        const uint32_t sg = J.spp_offset + si;
-        const unsigned long long path = static_cast<unsigned long long>(sg) * J.npix + pix;
-        float sx, sy;
-        if (J.sampler == SPT_PIXEL_UNIFORM) {  // uniform_pixel_sampler.cpp:7-10
+// Camera path g into slot i: origin + pixel, direction + sample index, throughput + job / depth, radiance.
+__device__ __forceinline__ void new_path(const Wave& W, unsigned long long g, const PathBuf& to, uint32_t i) {
+    const uint32_t j = job_of(W, g);
+    const PtJob& J = W.jobs[j];
+    const unsigned long long lg = g - J.first;
+    const uint32_t sr = static_cast<uint32_t>(lg / J.npix);
+    const uint32_t pix = static_cast<uint32_t>(lg - static_cast<unsigned long long>(sr) * J.npix);
+    const uint32_t si = J.s_begin + sr;   // sample index within the pixel's spp
+    const uint32_t xx = pix % J.cam.vp_width, yy = pix / J.cam.vp_width;
+    const uint32_t x = J.cam.vp_left + xx, y = J.cam.vp_top + yy;
+    const uint32_t sg = J.spp_offset + si;
+    const unsigned long long path = static_cast<unsigned long long>(sg) * J.npix + pix;
+    float sx, sy;
+    if (J.sampler == SPT_PIXEL_UNIFORM) {  // uniform_pixel_sampler.cpp:7-10
+        Stream cs(J.seed, path, 0);
+        sx = cs.next();
+        sy = cs.next();
+    } else {
+        const uint32_t a = si / J.nsub, b = si % J.nsub;
+        if (J.sampler == SPT_PIXEL_REGULAR) {  // regular_pixel_sampler.cpp:10-13
+            float off = J.sw * 0.5f;
+            sx = J.sw * a + off;
+            sy = J.sw * b + off;
+        } else {  // jittered_pixel_sampler.cpp:11-20
             Stream cs(J.seed, path, 0);
-            sx = cs.next();
-            sy = cs.next();
-        } else {
-            const uint32_t a = si / J.nsub, b = si % J.nsub;
-            if (J.sampler == SPT_PIXEL_REGULAR) {  // regular_pixel_sampler.cpp:10-13
-                float off = J.sw * 0.5f;
-                sx = J.sw * a + off;
-                sy = J.sw * b + off;
-            } else {  // jittered_pixel_sampler.cpp:11-20
-                Stream cs(J.seed, path, 0);
-                float u0 = cs.next(), u1 = cs.next();
-                sx = J.sw * a + J.sw * u0;
-                sy = J.sw * b + J.sw * u1;
-            }
+            float u0 = cs.next(), u1 = cs.next();
+            sx = J.sw * a + J.sw * u0;
+            sy = J.sw * b + J.sw * u1;
         }
-        V3 o, d;
-        camera_ray(J.cam, static_cast<float>(x) + sx, static_cast<float>(y) + sy, o, d);
-        const uint32_t slot = c.n_alive + i;
-        cur.o[slot] = make_float4(o.x, o.y, o.z, __uint_as_float(pix));
-        cur.d[slot] = make_float4(d.x, d.y, d.z, __uint_as_float(sg));
-        cur.b[slot] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(j << 16));
-        cur.l[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (cur.r) cur.r[slot] = make_uint4(kNoRec, kNoRec, kNoRec, kNoRec);
     }
+    V3 o, d;
+    camera_ray(J.cam, static_cast<float>(x) + sx, static_cast<float>(y) + sy, o, d);
+    to.o[i] = make_float4(o.x, o.y, o.z, __uint_as_float(pix));
+    to.d[i] = make_float4(d.x, d.y, d.z, __uint_as_float(sg));
+    to.b[i] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(j << 16));
+    to.l[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (to.r) to.r[i] = make_uint4(kNoRec, kNoRec, kNoRec, kNoRec);
+}
+
+// This iteration's new camera paths, behind the live ones.
+__global__ void __launch_bounds__(256) k_generate(const __grid_constant__ Wave W, const Counters* __restrict__ ctr,
+                                                  const __grid_constant__ PathBuf cur) {
+    const uint32_t n_alive = ctr->n_alive;
+    const unsigned long long next = ctr->next_path;
+    const uint32_t n = n_new_paths(W, n_alive, next);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        new_path(W, next + i, cur, n_alive + i);
 }
 
 // The guide's cache entry of a surface point: its cell in a cache_res^3 grid over the guide's box and
@@ -165,8 +187,7 @@ __device__ __forceinline__ float4 hit_record(const DevScene& S, const Hit1& h) {
 template <int TRAV>
 __global__ void __launch_bounds__(256) k_extend(Wave W, const Counters* __restrict__ ctr, PathBuf cur,
                                                 float4* __restrict__ hits, uint32_t* status) {
-    const Counters c = *ctr;
-    const uint32_t n = c.n_alive + n_new_paths(W, c);
+    const uint32_t n = n_slots(W, ctr);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 o = cur.o[i], d = cur.d[i];
         const DevScene& S = W.jobs[__float_as_uint(cur.b[i].w) >> 16].S;
@@ -212,8 +233,7 @@ __global__ void __launch_bounds__(128, 7) k_extend_df(const __grid_constant__ Wa
                                                    Counters* __restrict__ ctr, const __grid_constant__ PathBuf cur,
                                                    float4* __restrict__ hits, uint32_t* status) {
     __shared__ WarpQueue q[4];
-    const Counters c = *ctr;
-    const uint32_t n = c.n_alive + n_new_paths(W, c);
+    const uint32_t n = n_slots(W, ctr);
     PathRays<MANY> src{S, W, cur, hits, &S, wide_scene(S)};
     persistent_trace<DEPTH, false>(q[threadIdx.x >> 5], src, n, &ctr->fetch, static_cast<int>(W.stack_limit), status);
 }
@@ -230,62 +250,64 @@ __device__ __forceinline__ bool rec_live(uint32_t r, uint32_t gen) { return r !=
 
 // ---- shading grouped by material class (tune.sort_shading) ------------------------------------
 // A class is what decides the shade kernel's control flow: a miss, a layered stack, or the type of a
-// single-layer BSDF.  The slots of an iteration are counted per class, the counts turned into
-// offsets, and the slot indices scattered into `order`, so the warps of k_shade take the paths of one
-// class together.  The order is only a permutation of slots: every path computes the same values.
-constexpr int kShadeClasses = 8;   // miss, layered, 4 single-layer BSDF types (+ 2 spare)
+// single-layer BSDF.  A block orders a tile of slots by class (a counting sort in shared memory) before it
+// shades them, so its warps take the paths of one class together.  The order is only a permutation of
+// slots: every path computes the same values.  (Counting, scanning and scattering the slots of the whole
+// iteration took three kernels, two passes over the hits and contended global counters: with those and
+// the kernel that moved the counters, the layered scene rendered in 16.6 instead of 16.3 ms, a batch of
+// eight scenes in 17.1 instead of 14.7.)
+constexpr uint32_t kShadeClasses = 6;   // miss, layered, 4 single-layer BSDF types
+constexpr uint32_t kShadeTile = 1024;   // slots per tile at most: 32 groups of one warp's width
 
-__device__ __forceinline__ int shade_class(const Wave& W, const PathBuf& cur, const float4* hits, uint32_t i) {
-    const uint32_t prim = __float_as_uint(hits[i].y);
+__device__ __forceinline__ uint32_t shade_class(const Wave& W, const PathBuf& cur, const float4* hits, uint32_t i) {
+    const uint32_t prim = __float_as_uint(__ldg(&hits[i].y));
     if (prim == SPT_MISS) return 0;
-    const PtJob& J = W.jobs[__float_as_uint(cur.b[i].w) >> 16];
-    const DevMaterial m = J.S.mat[J.S.prim_mat[prim]];
-    if (m.layer_count != 1) return 1;
-    return 2 + (J.S.bsdf[J.S.layer_ids[m.layer_begin]].type & 3);
+    const DevScene& S = W.jobs[__float_as_uint(__ldg(&cur.b[i].w)) >> 16].S;
+    return static_cast<uint32_t>(S.mat[S.prim_mat[prim]].shade_class);
 }
 
-// counts[k] += slots of class k (block-local histogram, one atomic per class per block)
-__global__ void __launch_bounds__(256) k_class_count(Wave W, const Counters* __restrict__ ctr, PathBuf cur,
-                                                     const float4* __restrict__ hits, uint32_t* counts) {
-    __shared__ uint32_t h[kShadeClasses];
-    if (threadIdx.x < kShadeClasses) h[threadIdx.x] = 0;
-    __syncthreads();
-    const Counters c = *ctr;
-    const uint32_t n = c.n_alive + n_new_paths(W, c);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        atomicAdd(&h[shade_class(W, cur, hits, i)], 1u);
-    __syncthreads();
-    if (threadIdx.x < kShadeClasses && h[threadIdx.x]) atomicAdd(&counts[threadIdx.x], h[threadIdx.x]);
-}
+struct ShadeOrder {
+    uint16_t order[kShadeTile];         // tile slots by class
+    uint16_t key[kShadeTile];           // class << 8 | place among the group's slots of that class
+    uint16_t first[kShadeClasses][32];  // per class and group: its slots, then its first place
+};
 
-// cursors[k] = counts[0] + ... + counts[k-1]; counts cleared for the next iteration
-__global__ void k_class_offsets(uint32_t* counts, uint32_t* cursors) {
-    uint32_t sum = 0;
-    for (int k = 0; k < kShadeClasses; ++k) {
-        cursors[k] = sum;
-        sum += counts[k];
-        counts[k] = 0;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_class_scatter(Wave W, const Counters* __restrict__ ctr, PathBuf cur,
-                                                       const float4* __restrict__ hits, uint32_t* cursors,
-                                                       uint32_t* __restrict__ order) {
-    const Counters c = *ctr;
-    const uint32_t n = c.n_alive + n_new_paths(W, c);
-    const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const int k = i < n ? shade_class(W, cur, hits, i) : -1;
-        for (int q = 0; q < kShadeClasses; ++q) {   // warp-aggregated append per class
-            const unsigned mask = __ballot_sync(0xFFFFFFFFu, k == q);
-            if (!mask) continue;
-            uint32_t first = 0;
-            if (lane == __ffs(mask) - 1) first = atomicAdd(&cursors[q], static_cast<uint32_t>(__popc(mask)));
-            first = __shfl_sync(0xFFFFFFFFu, first, __ffs(mask) - 1);
-            if (k == q) order[first + __popc(mask & ((1u << lane) - 1u))] = i;
+// order[0 .. m) = the tile's slots base .. base + m - 1 by class (m <= kShadeTile), by the whole block.
+__device__ __forceinline__ void order_tile(ShadeOrder& so, const Wave& W, const PathBuf& cur, const float4* hits,
+                                           uint32_t base, uint32_t m) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const unsigned lt = (1u << lane) - 1u;
+    for (uint32_t k = threadIdx.x; k < kShadeClasses * 32; k += blockDim.x) so.first[k >> 5][k & 31u] = 0;
+    __syncthreads();   // also: the last tile's order has been read
+    for (uint32_t t = threadIdx.x; t - lane < m; t += blockDim.x) {   // whole warps
+        const uint32_t c = t < m ? shade_class(W, cur, hits, base + t) : kShadeClasses;
+        const unsigned same = __match_any_sync(0xFFFFFFFFu, c);
+        if (t < m) {
+            const uint32_t place = __popc(same & lt);
+            so.key[t] = static_cast<uint16_t>((c << 8) | place);
+            if (place == 0) so.first[c][t >> 5] = static_cast<uint16_t>(__popc(same));
         }
     }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        uint32_t sum = 0;
+        for (uint32_t c = 0; c < kShadeClasses; ++c) {
+            const uint32_t v = so.first[c][lane];
+            uint32_t x = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                if (lane >= static_cast<uint32_t>(o)) x += y;
+            }
+            so.first[c][lane] = static_cast<uint16_t>(sum + x - v);
+            sum += __shfl_sync(0xFFFFFFFFu, x, 31);
+        }
+    }
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < m; t += blockDim.x) {
+        const uint32_t k = so.key[t];
+        so.order[so.first[k >> 8][t >> 5] + (k & 0xFFu)] = static_cast<uint16_t>(t);
+    }
+    __syncthreads();
 }
 
 // Shading is latency-bound, so occupancy pays: at most 80 registers (three blocks of 256 threads per
@@ -295,21 +317,34 @@ __global__ void __launch_bounds__(256) k_class_scatter(Wave W, const Counters* _
 // RECORDS: the guided render still trains, so paths carry the ids of their open training records and
 // add the emission they find to them.  Once the guide is frozen (the last pass of a guided render,
 // nearly all of its samples) that state is neither read nor written.
-template <bool GUIDED, bool RECORDS>
-__global__ void __launch_bounds__(256, 3) k_shade(Wave W, Counters* __restrict__ ctr, PathBuf cur, PathBuf nxt,
-                                               const float4* __restrict__ hits, GuideIO G,
-                                               const uint32_t* __restrict__ order) {
-    const Counters c = *ctr;
-    const uint32_t n = c.n_alive + n_new_paths(W, c);
+// SORT: the slots of a tile in class order (above).
+// finish: after this iteration the render's device-side loop (a conditional WHILE node of the CUDA graph)
+// is told whether to go round again: unless every path has ended, or with the timeout status bit once
+// the iteration budget is spent.  The budget bounds the loop whatever the kernels before it did.
+template <bool GUIDED, bool RECORDS, bool SORT>
+__global__ void __launch_bounds__(256, 3) k_shade(const __grid_constant__ Wave W, Counters* __restrict__ ctr,
+                                               const __grid_constant__ PathBuf cur, const __grid_constant__ PathBuf nxt,
+                                               const float4* __restrict__ hits, const __grid_constant__ GuideIO G,
+                                               LoopEnd finish) {
+    __shared__ ShadeOrder so;   // SORT only
+    const uint32_t n = n_slots(W, ctr);
+    const uint32_t train_on = RECORDS ? ctr->train_on : 0u, rec_gen = RECORDS ? ctr->rec_gen : 0u;
     const uint32_t lane = threadIdx.x & 31;
+    // sorted tiles as large as still leaves every block one
+    const uint32_t tile = SORT ? min(kShadeTile, max(1u, (n + gridDim.x * blockDim.x - 1) / (gridDim.x * blockDim.x)) * blockDim.x)
+                               : blockDim.x;
+    for (uint32_t tbase = blockIdx.x * tile; tbase < n; tbase += gridDim.x * tile) {
+    const uint32_t m = min(tile, n - tbase);
+    if (SORT) order_tile(so, W, cur, hits, tbase, m);
     // all lanes of a warp iterate together so the append below can be warp-aggregated
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t j = base + threadIdx.x;
+    for (uint32_t off = 0; off < m; off += blockDim.x) {
+        const uint32_t t = off + threadIdx.x;
+        const bool valid = t < m;
         bool keep = false;
         float4 wo_o, wo_d, wo_b, wo_l;
         uint4 rr = make_uint4(kNoRec, kNoRec, kNoRec, kNoRec);
-        if (j < n) {
-            const uint32_t i = order ? order[j] : j;   // the slot this lane shades
+        if (valid) {
+            const uint32_t i = tbase + (SORT ? so.order[t] : t);   // the slot this lane shades
             // the slot's last use in this iteration (the buffer is rewritten as the next one's output):
             // evict-first loads leave L2 to the scene
             const float4 o4 = __ldcs(cur.o + i), d4 = __ldcs(cur.d + i), b4 = __ldcs(cur.b + i), l4 = __ldcs(cur.l + i),
@@ -379,7 +414,7 @@ __global__ void __launch_bounds__(256, 3) k_shade(Wave W, Counters* __restrict__
                     const V3 add = beta * le;
                     const uint32_t ids[4] = {rr.x, rr.y, rr.z, rr.w};
                     for (int k = 0; k < 4; ++k)
-                        if (rec_live(ids[k], c.rec_gen)) {
+                        if (rec_live(ids[k], rec_gen)) {
                             float4* sx = G.recx + 2ull * (ids[k] & 0xFFFFFFu) + 1;
                             const float4 v = *sx;
                             *sx = make_float4(v.x + add.x, v.y + add.y, v.z + add.z, 0.0f);
@@ -401,7 +436,7 @@ __global__ void __launch_bounds__(256, 3) k_shade(Wave W, Counters* __restrict__
                         (GUIDED && !(isfinite(beta.x) && isfinite(beta.y) && isfinite(beta.z)))) {
                         done = true;
                     } else {
-                        if (GUIDED && RECORDS && gi != kNoRec && c.train_on) {
+                        if (GUIDED && RECORDS && gi != kNoRec && train_on) {
                             const uint32_t r = atomicAdd(&ctr->rec_count, 1u);
                             if (r < G.rec_cap) {
                                 G.rec[4ull * r] = make_float4(pos.x, pos.y, pos.z, 0.0f);
@@ -410,7 +445,7 @@ __global__ void __launch_bounds__(256, 3) k_shade(Wave W, Counters* __restrict__
                                 G.rec[4ull * r + 3] = make_float4(wwi.x, wwi.y, wwi.z, 0.0f);
                                 G.recx[2ull * r] = make_float4(beta0.x, beta0.y, beta0.z, 0.0f);
                                 G.recx[2ull * r + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                                rr = make_uint4(((c.rec_gen & 0xFFu) << 24) | r, rr.x, rr.y, rr.z);
+                                rr = make_uint4(((rec_gen & 0xFFu) << 24) | r, rr.x, rr.y, rr.z);
                             }
                         }
                         keep = true;
@@ -423,13 +458,13 @@ __global__ void __launch_bounds__(256, 3) k_shade(Wave W, Counters* __restrict__
             }
             if (done) splat(J, pix, L);
         }
-        const unsigned mask = __ballot_sync(0xFFFFFFFFu, keep);
-        if (mask) {
+        const unsigned kept = __ballot_sync(0xFFFFFFFFu, keep);
+        if (kept) {
             uint32_t first = 0;
-            if (lane == 0) first = atomicAdd(&ctr->n_next, static_cast<uint32_t>(__popc(mask)));
+            if (lane == 0) first = atomicAdd(&ctr->n_next, static_cast<uint32_t>(__popc(kept)));
             first = __shfl_sync(0xFFFFFFFFu, first, 0);
             if (keep) {
-                const uint32_t slot = first + __popc(mask & ((1u << lane) - 1u));
+                const uint32_t slot = first + __popc(kept & ((1u << lane) - 1u));
                 nxt.o[slot] = wo_o;
                 nxt.d[slot] = wo_d;
                 nxt.b[slot] = wo_b;
@@ -438,30 +473,31 @@ __global__ void __launch_bounds__(256, 3) k_shade(Wave W, Counters* __restrict__
             }
         }
     }
-}
-
-__global__ void k_advance(Wave W, Counters* ctr) {
-    Counters c = *ctr;
-    const uint32_t n_new = n_new_paths(W, c);
-    c.segments += c.n_alive + n_new;
-    c.next_path += n_new;
-    c.n_alive = c.n_next;
-    c.n_next = 0;
-    c.fetch = 0;
-    c.iterations += 1;
-    *ctr = c;
-}
-
-// End of one pass of the render's device-side loop (a conditional WHILE node of the CUDA graph): loop
-// again unless every path has ended, or stop with the timeout status bit once the iteration budget
-// is spent.  The budget bounds the loop whatever the kernels before it did.
-__global__ void k_continue(Wave W, const Counters* __restrict__ ctr, uint32_t max_iter, uint32_t* status,
-                           cudaGraphConditionalHandle loop) {
-    const Counters c = *ctr;
-    const bool done = c.next_path >= W.total && c.n_alive == 0;
-    const bool spent = !done && c.iterations >= max_iter;
-    if (spent) atomicOr(status, 4u);
-    cudaGraphSetConditional(loop, (done || spent) ? 0u : 1u);
+    }
+    // the last block to finish moves the counters: every block has read them and done its appends
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&ctr->done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            volatile Counters* v = ctr;
+            const unsigned long long next = v->next_path + (n - v->n_alive);
+            const uint32_t alive = v->n_next, iterations = v->iterations + 1;
+            v->next_path = next;
+            v->segments += n;
+            v->n_alive = alive;
+            v->n_next = 0;
+            v->fetch = 0;
+            v->iterations = iterations;
+            v->done = 0;
+            if (finish.on) {
+                const bool ended = next >= W.total && alive == 0;
+                const bool spent = !ended && iterations >= finish.max_iterations;
+                if (spent) atomicOr(finish.status, 4u);
+                cudaGraphSetConditional(finish.loop, (ended || spent) ? 0u : 1u);
+            }
+        }
+    }
 }
 
 // Training weight of every record: luminance of (radiance gathered after the record / throughput at it),
@@ -597,9 +633,7 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
     void* mem;
     const size_t buf_bytes = stride * sizeof(float4);
     const size_t job_bytes = jobs.size() * sizeof(PtJob);
-    const size_t order_bytes = (stride * sizeof(uint32_t) + 255) & ~static_cast<size_t>(255);
-    if ((st = scratch(ctx, 5, buf_bytes * 9 + sizeof(Counters) + job_bytes + 512 + order_bytes + 256, &mem)) != SPT_OK)
-        return st;
+    if ((st = scratch(ctx, 5, buf_bytes * 9 + 256 + job_bytes, &mem)) != SPT_OK) return st;
     char* base = static_cast<char*>(mem);
     PathBuf A{reinterpret_cast<float4*>(base), reinterpret_cast<float4*>(base + buf_bytes),
               reinterpret_cast<float4*>(base + 2 * buf_bytes), reinterpret_cast<float4*>(base + 3 * buf_bytes), nullptr};
@@ -609,15 +643,14 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
     float4* hits = reinterpret_cast<float4*>(base + 8 * buf_bytes);
     Counters* d_ctr = reinterpret_cast<Counters*>(base + 9 * buf_bytes);
     PtJob* d_jobs = reinterpret_cast<PtJob*>(base + 9 * buf_bytes + 256);
-    char* tail = base + 9 * buf_bytes + 256 + ((job_bytes + 255) & ~static_cast<size_t>(255));
-    uint32_t* d_order = reinterpret_cast<uint32_t*>(tail);
-    uint32_t* d_class = reinterpret_cast<uint32_t*>(tail + order_bytes);   // counts[8], cursors[8]
+    static_assert(sizeof(Counters) <= 256, "the job table follows the counters");
     bool any_layered = false;
     for (const PtJob& J : jobs) any_layered |= J.layered != 0;
     // measured: +8 % on the layered 1.3M-tri workload, -6 % on the box of Lambertian walls
     const bool sort_shading = tune.sort_shading == 1 || (tune.sort_shading == 0 && any_layered);
-    SPT_CUDA(ctx, cudaMemsetAsync(d_ctr, 0, sizeof(Counters), ctx->stream));
-    if (sort_shading) SPT_CUDA(ctx, cudaMemsetAsync(d_class, 0, 2 * kShadeClasses * sizeof(uint32_t), ctx->stream));
+    Counters init{};
+    init.train_on = guide && train_budget > 0 ? 1u : 0u;
+    SPT_CUDA(ctx, cudaMemcpyAsync(d_ctr, &init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
     SPT_CUDA(ctx, cudaMemcpyAsync(d_jobs, jobs.data(), job_bytes, cudaMemcpyHostToDevice, ctx->stream));
     GuideIO G{};
     uint32_t batch = 0, rec_cap = 0;
@@ -647,9 +680,6 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
             G.lo[k] = guide->model.lo[k];
             G.inv_ext[k] = guide->model.inv_ext[k];
         }
-        const uint32_t on = train_budget > 0 ? 1u : 0u;
-        SPT_CUDA(ctx, cudaMemcpyAsync(&d_ctr->train_on, &on, sizeof(on), cudaMemcpyHostToDevice, ctx->stream));
-        SPT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
     Counters* h_ctr;
     if ((st = pinned(ctx, sizeof(Counters), reinterpret_cast<void**>(&h_ctr))) != SPT_OK) return st;
@@ -689,33 +719,26 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
     // Only a guide that trains during the render needs the host between iterations (it runs the
     // optimiser steps on the records the paths wrote), or a caller that asks for the host-driven loop
     // (tune.host_loop).  Every other render is one launch of a graph whose WHILE node repeats two
-    // iterations until k_continue sees the pool drained.
+    // iterations until k_shade's last block sees the pool drained.
     const bool host_loop = (guide && train_budget > 0) || tune.host_loop != 0;
+    auto shade = sort_shading ? (!guide            ? k_shade<false, false, true>
+                                 : train_budget > 0 ? k_shade<true, true, true>
+                                                    : k_shade<true, false, true>)
+                              : (!guide            ? k_shade<false, false, false>
+                                 : train_budget > 0 ? k_shade<true, true, false>
+                                                    : k_shade<true, false, false>);
     auto record_iterations = [&](cudaGraphConditionalHandle* loop) {
         for (int it = 0; it < 2; ++it) {
             PathBuf& cur = it ? B : A;
             PathBuf& nxt = it ? A : B;
-            k_generate<<<g_gen, 256, 0, ctx->stream>>>(W, d_ctr, cur);
+            if (total > cap) k_generate<<<g_gen, 256, 0, ctx->stream>>>(W, d_ctr, cur);
             if (trav == 2) ext_df<<<g_df, 128, 0, ctx->stream>>>(W, *one, d_ctr, cur, hits, ctx->d_status);
             else if (trav == 1) k_extend<1><<<g_ext, eb, 0, ctx->stream>>>(W, d_ctr, cur, hits, ctx->d_status);
             else k_extend<0><<<g_ext, eb, 0, ctx->stream>>>(W, d_ctr, cur, hits, ctx->d_status);
-            const uint32_t* order = nullptr;
-            if (sort_shading) {
-                k_class_count<<<g_shd, 256, 0, ctx->stream>>>(W, d_ctr, cur, hits, d_class);
-                k_class_offsets<<<1, 1, 0, ctx->stream>>>(d_class, d_class + kShadeClasses);
-                k_class_scatter<<<g_shd, 256, 0, ctx->stream>>>(W, d_ctr, cur, hits, d_class + kShadeClasses, d_order);
-                order = d_order;
-            }
-            if (guide) {
-                if (train_budget > 0) k_shade<true, true><<<g_shd, sb, 0, ctx->stream>>>(W, d_ctr, cur, nxt, hits, G, order);
-                else k_shade<true, false><<<g_shd, sb, 0, ctx->stream>>>(W, d_ctr, cur, nxt, hits, G, order);
-            } else {
-                k_shade<false, false><<<g_shd, sb, 0, ctx->stream>>>(W, d_ctr, cur, nxt, hits, G, order);
-            }
-            k_advance<<<1, 1, 0, ctx->stream>>>(W, d_ctr);
+            LoopEnd finish{};
+            if (loop && it) finish = LoopEnd{1u, static_cast<uint32_t>(max_iter), ctx->d_status, *loop};
+            shade<<<g_shd, sb, 0, ctx->stream>>>(W, d_ctr, cur, nxt, hits, G, finish);
         }
-        if (loop)
-            k_continue<<<1, 1, 0, ctx->stream>>>(W, d_ctr, static_cast<uint32_t>(max_iter), ctx->d_status, *loop);
     };
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -762,6 +785,8 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
         return cuda_fail(ctx, ce, "cudaGraphInstantiate");
     }
     SPT_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
+    // a pool that holds every camera path is filled once, before the loop
+    if (total <= cap) k_generate<<<g_gen, 256, 0, ctx->stream>>>(W, d_ctr, A);
     const unsigned check = std::max(1u, tune.check_every / 2);
     uint64_t it = 0;
     bool done = false;

@@ -37,7 +37,7 @@ struct DevBsdf {
 struct DevMaterial {
     int layer_begin, layer_count;
     float er, eg, eb;
-    float pad;
+    int shade_class;   // what decides the shade kernel's control flow: 1 a layered stack, 2 + type a single BSDF
 };
 
 struct DevScene {

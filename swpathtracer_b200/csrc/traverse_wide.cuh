@@ -517,7 +517,7 @@ __device__ __forceinline__ void persistent_trace(WarpQueue& Q, Source& src, uint
             const uint32_t pool = Q.pool, have = Q.pool_end - pool;
             const uint32_t cnt = __popc(wants), rank = __popc(wants & lt);
             uint32_t fresh = 0, extra = 0;
-            if (have < cnt) {
+            if (have < cnt && Q.first < n) {
                 unsigned long long f = 0;
                 if (lane == 0) f = atomicAdd(next, static_cast<unsigned long long>(kChunk));
                 f = __shfl_sync(0xFFFFFFFFu, f, 0) + Q.first;
