@@ -425,7 +425,6 @@ spt_status spt_scene_create(spt_context* ctx, const spt_scene_desc* d, const spt
         std::vector<float4> pair;
         std::vector<int2> leaf;
         std::vector<float> leaf_box;
-        std::vector<spt_bvh2_node> node2;
         if (tree) {
             const auto& nodes = tree->nodes;
             const size_t nn = nodes.size();
@@ -453,12 +452,11 @@ spt_status spt_scene_create(spt_context* ctx, const spt_scene_desc* d, const spt
                         p[0] = make_float4(L.min[0], L.min[1], L.min[2], L.max[0]);
                         p[1] = make_float4(L.max[1], L.max[2], R.min[0], R.min[1]);
                         p[2] = make_float4(R.min[2], R.max[0], R.max[1], R.max[2]);
-                        int4 refs = make_int4(ord[i + 1], ord[nd.right], 0, 0);
+                        int4 refs = make_int4(ord[i + 1], ord[nd.right], static_cast<int>(L.count), static_cast<int>(R.count));
                         std::memcpy(&p[3], &refs, sizeof(refs));
                     }
                 }
             });
-            node2 = nodes;
             S.n_inner = n_inner;
             S.n_leaves = n_leaf;
             S.n_nodes2 = static_cast<uint32_t>(nn);
@@ -576,7 +574,6 @@ spt_status spt_scene_create(spt_context* ctx, const spt_scene_desc* d, const spt
         up.add(pair, &S.pair);
         up.add(leaf, &S.leaf);
         up.add(leaf_box, &S.leaf_box);
-        up.add(node2, &S.node2);
         up.add(face, &S.face_normal);
         up.add(smooth, &S.smooth_normal);
         up.add(pm, &S.prim_mat);

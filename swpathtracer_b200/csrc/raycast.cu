@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kBlock) k_intersect(DevScene S, const float* _
     hits[i] = o;
 }
 
-template <int STRIDE>
+template <int STRIDE, bool FULL>
 __global__ void __launch_bounds__(kBlock) k_count(DevScene S, const float* __restrict__ rays, uint64_t n,
                                                   spt_hit* __restrict__ ref_hits, uint32_t* __restrict__ tests,
                                                   uint32_t* __restrict__ nhits, uint32_t* __restrict__ prim_tests,
@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(kBlock) k_count(DevScene S, const float* __res
     V3 ro, rd;
     load_ray<STRIDE, false>(rays, i, ro, rd);
     CountOut c;
-    Hit1 h = count_traverse<kStack>(S, ro, rd, c, status);
-    if (ref_hits) {
+    Hit1 h = count_traverse<kStack, FULL>(S, ro, rd, c, status);
+    if (FULL && ref_hits) {
         spt_hit o;
         o.t = h.t;
         o.prim_id = h.found ? slot_prim(S, h.slot) : SPT_MISS;
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kBlock) k_count(DevScene S, const float* __res
         ref_hits[i] = o;
     }
     if (tests) tests[i] = c.tests;
-    if (nhits) nhits[i] = c.hits;
+    if (FULL && nhits) nhits[i] = c.hits;
     if (prim_tests) prim_tests[i] = c.prim_tests;
 }
 
@@ -172,7 +172,9 @@ __device__ __forceinline__ void tile_pixel(uint32_t& x, uint32_t& y) {
     y = blockIdx.y * 16 + (w >> 1) * 4 + (lane >> 3);
 }
 
-template <int MODE, int TRAV>
+// STATS: the image's statistics (tests and passes of the reference's own traversal, which gives the hit
+// as well).
+template <int MODE, int TRAV, bool STATS>
 __global__ void __launch_bounds__(256) k_raycast(DevScene S, DevCamera cam, void* __restrict__ out,
                                                  StatAcc* stats, uint32_t* status) {
     uint32_t x, y;
@@ -183,9 +185,13 @@ __global__ void __launch_bounds__(256) k_raycast(DevScene S, DevCamera cam, void
         V3 o, d;
         camera_ray(cam, static_cast<float>(x) + 0.5f, static_cast<float>(y) + 0.5f, o, d);
         const uint64_t idx = static_cast<uint64_t>(y) * cam.width + x;
-        if (MODE == SPT_RAYCAST_COUNT || stats) {
+        if (MODE == SPT_RAYCAST_COUNT && !STATS) {
             CountOut c;
-            Hit1 h = count_traverse<kStack>(S, o, d, c, status);
+            count_traverse<kStack, false>(S, o, d, c, status);
+            static_cast<long long*>(out)[idx] = static_cast<long long>(c.tests);
+        } else if (STATS) {
+            CountOut c;
+            Hit1 h = count_traverse<kStack, true>(S, o, d, c, status);
             tests = c.tests;
             hits = c.hits;
             if (MODE == SPT_RAYCAST_COUNT) {
@@ -216,7 +222,7 @@ __global__ void __launch_bounds__(256) k_raycast(DevScene S, DevCamera cam, void
             }
         }
     }
-    if (stats) reduce_stats(stats, valid, tests, hits);
+    if (STATS) reduce_stats(stats, valid, tests, hits);
 }
 
 inline unsigned blocks_for(uint64_t n, int block) { return static_cast<unsigned>((n + block - 1) / block); }
@@ -345,12 +351,10 @@ spt_status launch_count(spt_context* ctx, const spt_scene* sc, const float* d_ra
                         uint32_t* d_tests, uint32_t* d_hits, uint32_t* d_prim_tests, cudaStream_t s, int stride) {
     if (n == 0) return SPT_OK;
     if (n > (1ull << 36)) return fail(ctx, SPT_ERR_INVALID_ARGUMENT, "too many rays in one call");
-    if (stride == 6)
-        k_count<6><<<blocks_for(n, kBlock), kBlock, 0, s>>>(sc->dev, d_rays, n, d_ref_hits, d_tests, d_hits,
-                                                            d_prim_tests, ctx->d_status);
-    else
-        k_count<8><<<blocks_for(n, kBlock), kBlock, 0, s>>>(sc->dev, d_rays, n, d_ref_hits, d_tests, d_hits,
-                                                            d_prim_tests, ctx->d_status);
+    // the test counts alone need no primitive tested
+    const bool full = d_ref_hits || d_hits;
+    auto k = stride == 6 ? (full ? k_count<6, true> : k_count<6, false>) : (full ? k_count<8, true> : k_count<8, false>);
+    k<<<blocks_for(n, kBlock), kBlock, 0, s>>>(sc->dev, d_rays, n, d_ref_hits, d_tests, d_hits, d_prim_tests, ctx->d_status);
     SPT_CUDA(ctx, cudaGetLastError());
     return SPT_OK;
 }
@@ -359,15 +363,15 @@ static spt_status launch_raycast(spt_context* ctx, const spt_scene* sc, const De
                                  StatAcc* d_stats, cudaStream_t s) {
     dim3 grid((cam.width + 15) / 16, (cam.height + 15) / 16);
     const bool w = sc->dev.traversal >= 1;
-    if (mode == SPT_RAYCAST_NORMAL) {
-        if (w) k_raycast<SPT_RAYCAST_NORMAL, 1><<<grid, 256, 0, s>>>(sc->dev, cam, d_out, d_stats, ctx->d_status);
-        else k_raycast<SPT_RAYCAST_NORMAL, 0><<<grid, 256, 0, s>>>(sc->dev, cam, d_out, d_stats, ctx->d_status);
-    } else if (mode == SPT_RAYCAST_DEPTH) {
-        if (w) k_raycast<SPT_RAYCAST_DEPTH, 1><<<grid, 256, 0, s>>>(sc->dev, cam, d_out, d_stats, ctx->d_status);
-        else k_raycast<SPT_RAYCAST_DEPTH, 0><<<grid, 256, 0, s>>>(sc->dev, cam, d_out, d_stats, ctx->d_status);
-    } else {
-        k_raycast<SPT_RAYCAST_COUNT, 0><<<grid, 256, 0, s>>>(sc->dev, cam, d_out, d_stats, ctx->d_status);
-    }
+    auto k = mode == SPT_RAYCAST_NORMAL  ? (d_stats ? k_raycast<SPT_RAYCAST_NORMAL, 0, true>
+                                            : w     ? k_raycast<SPT_RAYCAST_NORMAL, 1, false>
+                                                    : k_raycast<SPT_RAYCAST_NORMAL, 0, false>)
+             : mode == SPT_RAYCAST_DEPTH ? (d_stats ? k_raycast<SPT_RAYCAST_DEPTH, 0, true>
+                                            : w     ? k_raycast<SPT_RAYCAST_DEPTH, 1, false>
+                                                    : k_raycast<SPT_RAYCAST_DEPTH, 0, false>)
+                                         : (d_stats ? k_raycast<SPT_RAYCAST_COUNT, 0, true>
+                                                    : k_raycast<SPT_RAYCAST_COUNT, 0, false>);
+    k<<<grid, 256, 0, s>>>(sc->dev, cam, d_out, d_stats, ctx->d_status);
     SPT_CUDA(ctx, cudaGetLastError());
     return SPT_OK;
 }

@@ -22,9 +22,8 @@ namespace spt {
 //                               sphere:   {centre, prim id} {radius, 0, 0, leaf id} {0, 0, 0, type}
 //   pair[4*i .. 4*i+3]        one 64-byte record per inner node i (pre-order ordinal): both
 //                             children's boxes + child refs (>= 0 inner ordinal, < 0 ~leaf id)
+//                             + a leaf child's primitive count (0 for an inner child)
 //   leaf[l]                   {first slot, count} of leaf l; leaf_box[l] its box (inside test)
-//   node2[]                   the flattened binary tree (spt_bvh2_node), for the exhaustive
-//                             reference-order traversal that counts tests
 // ---------------------------------------------------------------------------------------------
 struct DevBsdf {
     int type, sampler;
@@ -45,7 +44,6 @@ struct DevScene {
     const float4* pair;
     const int2* leaf;
     const float* leaf_box;      // 6 floats per leaf
-    const spt_bvh2_node* node2;
     const float4* face_normal;  // per primitive (flat triangles)
     const float4* smooth_normal;  // 3 per primitive, or null
     const uint32_t* prim_mat;

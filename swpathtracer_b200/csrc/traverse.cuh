@@ -11,9 +11,10 @@
 //   every non-root box is its primitives' bounds inflated by 1e-3, so any hit inside one lies
 //   at least 1e-3 / |d_axis| past the box's entry and before its exit.
 //
-// count_traverse(): the reference's traversal itself -- no ordering, no pruning -- over the
-//   flattened binary tree, counting box and primitive tests and passes
-//   (num_intersection_tests / num_intersections, sbvh.cpp:478-510), plus the hit it finds.
+// count_traverse(): the reference's exhaustive traversal -- no pruning -- counting box and primitive
+//   tests and passes (num_intersection_tests / num_intersections, sbvh.cpp:478-510), plus the hit it
+//   finds.  The counts are sums over the boxes whose parent's box passes, and the hit is the smallest
+//   (t, depth-first slot) that passes the inside test, so neither depends on the order.
 #pragma once
 
 #include "spt_device.cuh"
@@ -130,7 +131,30 @@ struct CountOut {
     uint32_t tests, hits, prim_tests;
 };
 
-template <int STACK>
+// The primitives first .. first + n - 1 of a passing leaf with box bx (NULL: no inside test).
+__device__ __forceinline__ void count_leaf(const DevScene& S, uint32_t first, uint32_t n, const float* bx, V3 o, V3 d,
+                                           CountOut& c, Hit1& h) {
+    for (uint32_t k = 0; k < n; ++k) {
+        const uint32_t s = first + k;
+        const float4 a = __ldg(S.tri + 3 * s), b = __ldg(S.tri + 3 * s + 1), cc = __ldg(S.tri + 3 * s + 2);
+        float t, u = 0.0f, v = 0.0f;
+        bool sphere = __float_as_int(cc.w) == SPT_PRIM_SPHERE;
+        bool ok = sphere ? sphere_test(f3v(a), b.x, o, d, t) : tri_test(f3v(a), f3v(b), f3v(cc), o, d, t, u, v);
+        if (!ok) continue;
+        ++c.hits;
+        if (!(t > 0.0f) || !(t < h.t || (h.found && t == h.t && s < h.slot))) continue;
+        if (bx && !inside(bx, hit_pos(sphere, o, d, t))) continue;
+        h.t = t; h.u = u; h.v = v; h.slot = s; h.found = true;
+    }
+}
+
+// FULL: the primitives are tested, for the passes among them and the hit; without it c.hits counts boxes
+// only and no hit is returned (a test is counted whatever it finds, so the count of tests needs none).
+// A step visits a pair node: both children's boxes and, for a leaf child, its primitive count, in one
+// 64-byte record.  What bounds the traversal is its chain of dependent node loads and the boxes' slab
+// tests; a step per box, from the tree's own 32-byte nodes, and with the primitives tested for counts
+// that do not need them, took COUNT_BEFORE.
+template <int STACK, bool FULL>
 __device__ __forceinline__ Hit1 count_traverse(const DevScene& S, V3 o, V3 d, CountOut& c, uint32_t* overflow) {
     Hit1 h;
     h.t = inf_f();
@@ -141,58 +165,60 @@ __device__ __forceinline__ Hit1 count_traverse(const DevScene& S, V3 o, V3 d, Co
     c.tests = c.hits = c.prim_tests = 0;
     if (S.empty) return h;
     if (S.no_accel) {
-        for (uint32_t s = 0; s < S.n_prims; ++s) {
-            ++c.tests;
-            ++c.prim_tests;
-            const float4 a = __ldg(S.tri + 3 * s), b = __ldg(S.tri + 3 * s + 1), cc = __ldg(S.tri + 3 * s + 2);
-            float t, u = 0.0f, v = 0.0f;
-            bool sphere = __float_as_int(cc.w) == SPT_PRIM_SPHERE;
-            bool ok = sphere ? sphere_test(f3v(a), b.x, o, d, t) : tri_test(f3v(a), f3v(b), f3v(cc), o, d, t, u, v);
-            if (!ok) continue;
-            ++c.hits;
-            if ((t < h.t) && (t > 0.0f)) {
-                h.t = t; h.u = u; h.v = v; h.slot = s; h.found = true;
-            }
-        }
+        c.tests = c.prim_tests = S.n_prims;
+        if (FULL) count_leaf(S, 0, S.n_prims, nullptr, o, d, c, h);
         return h;
     }
     const RayInv r = ray_inv(o, d);
-    uint32_t stack[STACK];
-    int sp = 0;
-    stack[sp++] = 0;
-    while (sp > 0) {
-        const uint32_t i = stack[--sp];
-        const spt_bvh2_node nd = S.node2[i];
-        ++c.tests;
-        float t0, t1;
-        if (!slab(r, nd.min[0], nd.min[1], nd.min[2], nd.max[0], nd.max[1], nd.max[2], t0, t1)) continue;
-        ++c.hits;
-        if (nd.count) {
-            for (uint32_t k = 0; k < nd.count; ++k) {
-                const uint32_t s = nd.right + k;
-                ++c.tests;
-                ++c.prim_tests;
-                const float4 a = __ldg(S.tri + 3 * s), b = __ldg(S.tri + 3 * s + 1), cc = __ldg(S.tri + 3 * s + 2);
-                float t, u = 0.0f, v = 0.0f;
-                bool sphere = __float_as_int(cc.w) == SPT_PRIM_SPHERE;
-                bool ok = sphere ? sphere_test(f3v(a), b.x, o, d, t) : tri_test(f3v(a), f3v(b), f3v(cc), o, d, t, u, v);
-                if (!ok) continue;
-                ++c.hits;
-                if ((t > 0.0f) && (t < h.t)) {
-                    float bx[6] = {nd.min[0], nd.min[1], nd.min[2], nd.max[0], nd.max[1], nd.max[2]};
-                    if (inside(bx, hit_pos(sphere, o, d, t))) {
-                        h.t = t; h.u = u; h.v = v; h.slot = s; h.found = true;
-                    }
-                }
+    float t0, t1;
+    c.tests = 1;
+    if (!slab(r, S.root_min[0], S.root_min[1], S.root_min[2], S.root_max[0], S.root_max[1], S.root_max[2], t0, t1))
+        return h;
+    c.hits = 1;
+    if (S.root_is_leaf) {
+        const int2 fc = __ldg(S.leaf);
+        c.tests += fc.y;
+        c.prim_tests = fc.y;
+        if (FULL) count_leaf(S, fc.x, fc.y, S.leaf_box, o, d, c, h);
+        return h;
+    }
+    int stack[STACK];
+    int sp = 0, node = 0;
+    for (;;) {
+        const float4* p = S.pair + 4ull * node;
+        const float4 a = __ldg(p), b = __ldg(p + 1), e = __ldg(p + 2);
+        const int4 refs = __ldg(reinterpret_cast<const int4*>(p + 3));
+        const bool hl = slab(r, a.x, a.y, a.z, a.w, b.x, b.y, t0, t1), hr = slab(r, b.z, b.w, e.x, e.y, e.z, e.w, t0, t1);
+        c.tests += 2;
+        c.hits += (hl ? 1u : 0u) + (hr ? 1u : 0u);
+        if (hl && refs.x < 0) {
+            c.tests += refs.z;
+            c.prim_tests += refs.z;
+            if (FULL) {
+                const float bx[6] = {a.x, a.y, a.z, a.w, b.x, b.y};
+                count_leaf(S, __ldg(&S.leaf[~refs.x].x), refs.z, bx, o, d, c, h);
             }
-        } else if (sp + 2 <= STACK) {
-            stack[sp++] = nd.right;
-            stack[sp++] = i + 1;
+        }
+        if (hr && refs.y < 0) {
+            c.tests += refs.w;
+            c.prim_tests += refs.w;
+            if (FULL) {
+                const float bx[6] = {b.z, b.w, e.x, e.y, e.z, e.w};
+                count_leaf(S, __ldg(&S.leaf[~refs.y].x), refs.w, bx, o, d, c, h);
+            }
+        }
+        const bool il = hl && refs.x >= 0, ir = hr && refs.y >= 0;
+        if (il || ir) {
+            if (il && ir) {
+                if (sp < STACK) stack[sp++] = refs.y;
+                else atomicOr(overflow, 1u);
+            }
+            node = il ? refs.x : refs.y;
         } else {
-            atomicOr(overflow, 1u);
+            if (sp == 0) return h;
+            node = stack[--sp];
         }
     }
-    return h;
 }
 
 __device__ __forceinline__ uint32_t slot_prim(const DevScene& S, uint32_t slot) {
