@@ -215,6 +215,13 @@ struct PathRays {
         o = f3v(cur.o[i]);
         d = f3v(cur.d[i]);
     }
+    __device__ __forceinline__ void move(uint32_t from) {
+        if (!MANY) return;
+        auto get = [&](auto p) {
+            return reinterpret_cast<decltype(p)>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(p), from));
+        };
+        ws = WideScene{get(ws.wnode), get(ws.wtri), get(ws.leaf_box)};
+    }
     __device__ __forceinline__ const float* root_min() const { return MANY ? mine->root_min : S.root_min; }
     __device__ __forceinline__ const float* root_max() const { return MANY ? mine->root_max : S.root_max; }
     __device__ __forceinline__ WideScene scene() const { return MANY ? ws : wide_scene(S); }

@@ -50,6 +50,7 @@ struct RayBatch {
     __device__ __forceinline__ void load(uint32_t i, V3& o, V3& d) {
         load_ray<STRIDE, true>(rays, ORDERED ? __ldg(order + i) : i, o, d);
     }
+    __device__ __forceinline__ void move(uint32_t) {}
     __device__ __forceinline__ const float* root_min() const { return S.root_min; }
     __device__ __forceinline__ const float* root_max() const { return S.root_max; }
     __device__ __forceinline__ WideScene scene() const { return wide_scene(S); }
