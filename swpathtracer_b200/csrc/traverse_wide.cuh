@@ -713,6 +713,35 @@ __device__ __forceinline__ void persistent_trace(WarpQueue& Q, Source& src, uint
     }
 }
 
+// Closest hits of one ray per lane (valid lanes only), without refill: for rays that stay together on
+// their own (camera rays of a tile).
+template <int DEPTH, typename Source>
+__device__ __forceinline__ void trace_tile(WarpQueue& Q, Source& src, bool valid, V3 o, V3 d, uint32_t ray,
+                                           uint32_t* status) {
+    uint2 stack[DEPTH];
+    LaneTrace<DEPTH> tr;
+    tr.clear();
+    uint32_t qhead = 0, qtail = 0;
+    unsigned exact_lanes = 0;
+    if ((threadIdx.x & 31u) == 0) Q.tail = 0;
+    if (valid && !tr.start(src.root_min(), src.root_max(), o, d, Q, qhead)) src.store(ray, inf_f(), SPT_MISS, 0.0f, 0.0f);
+    __syncwarp();
+    for (;;) {
+        const bool fin = tr.has && !tr.walking() && static_cast<int>(qhead - tr.last) >= 0;
+        const unsigned ends = __ballot_sync(0xFFFFFFFFu, fin), busy = __ballot_sync(0xFFFFFFFFu, tr.has && !fin);
+        if (__popc(ends) >= kRefill || __popc(busy) <= kLast) {
+            if (fin) {
+                if (settle(Q, src, tr, ray)) tr.has = false;
+                else tr.restart(Q, qhead, true);
+            }
+            exact_lanes = __ballot_sync(0xFFFFFFFFu, tr.has && tr.exact);
+            if (__popc(__ballot_sync(0xFFFFFFFFu, tr.has)) <= kLast) break;
+        }
+        warp_step(Q, qhead, qtail, src.scene(), tr, stack, DEPTH, status, exact_lanes);
+    }
+    if (__any_sync(0xFFFFFFFFu, tr.has)) trace_last(Q, src, tr, stack, ray, qhead, qtail, DEPTH, status, exact_lanes);
+}
+
 // Closest hit with the traversal the scene selected (a kernel template parameter, so each kernel
 // carries one traversal's registers).
 template <int TRAV>
