@@ -82,13 +82,6 @@ struct GuideIO {
     float4* recx;          // 2 float4 per record: throughput at the record, radiance gathered after it
 };
 
-// What k_shade does at the end of an iteration that ends a pass of the device-side loop.
-struct LoopEnd {
-    uint32_t on, max_iterations;
-    uint32_t* status;
-    cudaGraphConditionalHandle loop;
-};
-
 constexpr uint32_t kNoRec = 0xFFFFFFFFu;
 constexpr uint32_t kRecBatches = 4;   // training records held per render: this many optimiser batches
 constexpr uint32_t kTrainEpochs = 4;  // optimiser passes over each filled record buffer
@@ -325,14 +318,10 @@ __device__ __forceinline__ void order_tile(ShadeOrder& so, const Wave& W, const 
 // add the emission they find to them.  Once the guide is frozen (the last pass of a guided render,
 // nearly all of its samples) that state is neither read nor written.
 // SORT: the slots of a tile in class order (above).
-// finish: after this iteration the render's device-side loop (a conditional WHILE node of the CUDA graph)
-// is told whether to go round again: unless every path has ended, or with the timeout status bit once
-// the iteration budget is spent.  The budget bounds the loop whatever the kernels before it did.
 template <bool GUIDED, bool RECORDS, bool SORT>
 __global__ void __launch_bounds__(256, 3) k_shade(const __grid_constant__ Wave W, Counters* __restrict__ ctr,
                                                const __grid_constant__ PathBuf cur, const __grid_constant__ PathBuf nxt,
-                                               const float4* __restrict__ hits, const __grid_constant__ GuideIO G,
-                                               LoopEnd finish) {
+                                               const float4* __restrict__ hits, const __grid_constant__ GuideIO G) {
     __shared__ ShadeOrder so;   // SORT only
     const uint32_t n = n_slots(W, ctr);
     const uint32_t train_on = RECORDS ? ctr->train_on : 0u, rec_gen = RECORDS ? ctr->rec_gen : 0u;
@@ -489,22 +478,27 @@ __global__ void __launch_bounds__(256, 3) k_shade(const __grid_constant__ Wave W
             __threadfence();
             volatile Counters* v = ctr;
             const unsigned long long next = v->next_path + (n - v->n_alive);
-            const uint32_t alive = v->n_next, iterations = v->iterations + 1;
             v->next_path = next;
             v->segments += n;
-            v->n_alive = alive;
+            v->n_alive = v->n_next;
             v->n_next = 0;
             v->fetch = 0;
-            v->iterations = iterations;
+            v->iterations += 1;
             v->done = 0;
-            if (finish.on) {
-                const bool ended = next >= W.total && alive == 0;
-                const bool spent = !ended && iterations >= finish.max_iterations;
-                if (spent) atomicOr(finish.status, 4u);
-                cudaGraphSetConditional(finish.loop, (ended || spent) ? 0u : 1u);
-            }
         }
     }
+}
+
+// End of one pass of the render's device-side loop (a conditional WHILE node of the CUDA graph): loop
+// again unless every path has ended, or stop with the timeout status bit once the iteration budget
+// is spent.  The budget bounds the loop whatever the kernels before it did.  (A kernel of its own: one
+// that sets a graph condition cannot be profiled, and k_shade should be.)
+__global__ void k_continue(Wave W, const Counters* __restrict__ ctr, uint32_t max_iter, uint32_t* status,
+                           cudaGraphConditionalHandle loop) {
+    const bool done = ctr->next_path >= W.total && ctr->n_alive == 0;
+    const bool spent = !done && ctr->iterations >= max_iter;
+    if (spent) atomicOr(status, 4u);
+    cudaGraphSetConditional(loop, (done || spent) ? 0u : 1u);
 }
 
 // Training weight of every record: luminance of (radiance gathered after the record / throughput at it),
@@ -730,7 +724,7 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
     // Only a guide that trains during the render needs the host between iterations (it runs the
     // optimiser steps on the records the paths wrote), or a caller that asks for the host-driven loop
     // (tune.host_loop).  Every other render whose paths outnumber the pool is one launch of a graph whose
-    // WHILE node repeats two iterations until k_shade's last block sees the pool drained.
+    // WHILE node repeats two iterations until k_continue sees the pool drained.
     const bool host_loop = (guide && train_budget > 0) || tune.host_loop != 0;
     auto shade = sort_shading ? (!guide            ? k_shade<false, false, true>
                                  : train_budget > 0 ? k_shade<true, true, true>
@@ -739,14 +733,14 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
                                  : train_budget > 0 ? k_shade<true, true, false>
                                                     : k_shade<true, false, false>);
     // one iteration, from buffer A to B (it even) or back
-    auto iteration = [&](uint64_t it, const LoopEnd& finish) {
+    auto iteration = [&](uint64_t it) {
         PathBuf& cur = (it & 1) ? B : A;
         PathBuf& nxt = (it & 1) ? A : B;
         if (total > cap) k_generate<<<g_gen, 256, 0, ctx->stream>>>(W, d_ctr, cur);
         if (trav == 2) ext_df<<<g_df, 128, 0, ctx->stream>>>(W, *one, d_ctr, cur, hits, ctx->d_status);
         else if (trav == 1) k_extend<1><<<g_ext, eb, 0, ctx->stream>>>(W, d_ctr, cur, hits, ctx->d_status);
         else k_extend<0><<<g_ext, eb, 0, ctx->stream>>>(W, d_ctr, cur, hits, ctx->d_status);
-        shade<<<g_shd, sb, 0, ctx->stream>>>(W, d_ctr, cur, nxt, hits, G, finish);
+        shade<<<g_shd, sb, 0, ctx->stream>>>(W, d_ctr, cur, nxt, hits, G);
     };
     auto finalize = [&]() -> spt_status {   // sums -> means, and the end of the timed region
         for (const PtJob& J : jobs) {
@@ -779,7 +773,7 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
         for (uint64_t it = 0, stop = known ? depth_limit : 8;;) {
             // (the budget is looked at after every second iteration, as in the device-side loop)
             const uint64_t end = known ? stop : std::min<uint64_t>(stop, (max_iter + 1) & ~1ull);
-            for (; it < end; ++it) iteration(it, LoopEnd{});
+            for (; it < end; ++it) iteration(it);
             SPT_CUDA(ctx, cudaMemcpyAsync(h_ctr, d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, ctx->stream));
             if (known && (st = finalize()) != SPT_OK) return st;
             if ((st = check_status(ctx)) != SPT_OK) return st;   // waits; a stack overflow
@@ -796,11 +790,9 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
         return SPT_OK;
     }
     auto record_iterations = [&](cudaGraphConditionalHandle* loop) {
-        for (int it = 0; it < 2; ++it) {
-            LoopEnd finish{};
-            if (loop && it) finish = LoopEnd{1u, static_cast<uint32_t>(max_iter), ctx->d_status, *loop};
-            iteration(it, finish);
-        }
+        for (int it = 0; it < 2; ++it) iteration(it);
+        if (loop)
+            k_continue<<<1, 1, 0, ctx->stream>>>(W, d_ctr, static_cast<uint32_t>(max_iter), ctx->d_status, *loop);
     };
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
