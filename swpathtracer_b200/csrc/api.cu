@@ -403,15 +403,17 @@ spt_status spt_scene_create(spt_context* ctx, const spt_scene_desc* d, const spt
             any_sphere |= d->prim_type[i] == SPT_PRIM_SPHERE;
         }
         if (any_smooth) smooth.resize(3ull * n);
+        if (d->n_materials > (1u << 30)) return fail(ctx, SPT_ERR_UNSUPPORTED, "more than 2^30 materials");
         parallel_for(n, [&](size_t a, size_t b) {
             for (size_t i = a; i < b; ++i) {
                 const float* p = d->prim_data + 9ull * i;
+                const float w = bits_f(d->prim_material[i] | static_cast<uint32_t>(d->prim_type[i]) << 30);
                 if (d->prim_type[i] == SPT_PRIM_SPHERE) {
-                    face[i] = make_float4(p[0], p[1], p[2], p[3]);
+                    face[i] = make_float4(p[0], p[1], p[2], w);
                 } else {
                     V3 v0 = v3(p[0], p[1], p[2]), v1 = v3(p[3], p[4], p[5]), v2 = v3(p[6], p[7], p[8]);
                     V3 nn = normalize(cross(v1 - v0, v2 - v0));  // triangle.cpp:6
-                    face[i] = make_float4(nn.x, nn.y, nn.z, 0.0f);
+                    face[i] = make_float4(nn.x, nn.y, nn.z, w);
                     if (d->prim_type[i] == SPT_PRIM_SMOOTH_TRIANGLE) {
                         const float* q = d->prim_normals + 9ull * i;
                         for (int k = 0; k < 3; ++k)
@@ -545,7 +547,7 @@ spt_status spt_scene_create(spt_context* ctx, const spt_scene_desc* d, const spt
             o.br = b.rgb[0] / kPi; o.bg = b.rgb[1] / kPi; o.bb = b.rgb[2] / kPi;  // lambertian.cpp:6
         }
         std::vector<DevMaterial> ms(d->n_materials);
-        std::vector<int> layers;
+        std::vector<DevBsdf> layers;
         bool any_em = false;
         for (uint32_t i = 0; i < d->n_materials; ++i) {
             const spt_material& m = d->materials[i];
@@ -553,15 +555,13 @@ spt_status spt_scene_create(spt_context* ctx, const spt_scene_desc* d, const spt
             std::memset(&o, 0, sizeof(o));
             o.layer_begin = static_cast<int>(layers.size());
             for (uint32_t k = d->layered_offsets[m.layered_bsdf]; k < d->layered_offsets[m.layered_bsdf + 1]; ++k)
-                layers.push_back(static_cast<int>(d->layered_bsdf_ids[k]));
+                layers.push_back(bs[d->layered_bsdf_ids[k]]);
             o.layer_count = static_cast<int>(layers.size()) - o.layer_begin;
             o.er = m.emission[0]; o.eg = m.emission[1]; o.eb = m.emission[2];
-            o.shade_class = o.layer_count != 1 ? 1 : 2 + bs[layers[o.layer_begin]].type;
+            o.shade_class = o.layer_count != 1 ? 1 : 2 + layers[o.layer_begin].type;
             sc->any_layered |= o.layer_count > 1;
             any_em |= (m.emission[0] != 0.0f || m.emission[1] != 0.0f || m.emission[2] != 0.0f);
         }
-        std::vector<uint32_t> pm(d->prim_material, d->prim_material + n);
-        std::vector<uint8_t> pt(d->prim_type, d->prim_type + n);
         S.has_spheres = any_sphere;
         sc->n_materials = d->n_materials;
         sc->any_emission = any_em;
@@ -574,13 +574,10 @@ spt_status spt_scene_create(spt_context* ctx, const spt_scene_desc* d, const spt
         up.add(pair, &S.pair);
         up.add(leaf, &S.leaf);
         up.add(leaf_box, &S.leaf_box);
-        up.add(face, &S.face_normal);
+        up.add(face, &S.surface);
         up.add(smooth, &S.smooth_normal);
-        up.add(pm, &S.prim_mat);
-        up.add(pt, &S.prim_type);
-        up.add(bs, &S.bsdf);
         up.add(ms, &S.mat);
-        up.add(layers, &S.layer_ids);
+        up.add(layers, &S.layer);
         up.add(raw, &wn);
         up.add(wtri, &S.wtri);
         if ((s = up.commit(sc.get())) != SPT_OK) return s;

@@ -18,14 +18,14 @@ namespace spt {
 // metal): guided through the walk's single-internal-bounce component (layered_t1 below).
 __device__ __forceinline__ bool coated(const DevScene& S, const DevMaterial& m) {
     if (m.layer_count != 2) return false;
-    return S.bsdf[S.layer_ids[m.layer_begin]].type == SPT_BSDF_SMOOTH_DIELECTRIC &&
-           S.bsdf[S.layer_ids[m.layer_begin + 1]].type == SPT_BSDF_COOK_TORRANCE;
+    return S.layer[m.layer_begin].type == SPT_BSDF_SMOOTH_DIELECTRIC &&
+           S.layer[m.layer_begin + 1].type == SPT_BSDF_COOK_TORRANCE;
 }
 
 __device__ __forceinline__ bool guidable(const DevScene& S, const DevMaterial& m) {
     if (coated(S, m)) return true;
     if (m.layer_count != 1) return false;
-    const int t = S.bsdf[S.layer_ids[m.layer_begin]].type;
+    const int t = S.layer[m.layer_begin].type;
     return t == SPT_BSDF_LAMBERTIAN || t == SPT_BSDF_COOK_TORRANCE;
 }
 
@@ -110,10 +110,11 @@ __device__ __forceinline__ CoatT1 coat_t1(const DevBsdf& top, const DevBsdf& bot
 // outcomes take that same weight and whose other outcomes take f cos / (pdf (1 - mix))
 // (coated_walk_weight).  The expectation is the walk's.  The shade kernel makes the technique choice
 // and runs the walk itself, so that one copy of the walk serves guided and plain vertices.
+template <typename St>
 __device__ __forceinline__ GuidedSample coated_guide_sample(const DevScene& S, const DevMaterial& m, const float* frame,
-                                                            V3 wo, const float* entry, float mix, Stream& s) {
-    const DevBsdf top = S.bsdf[S.layer_ids[m.layer_begin]];
-    const DevBsdf bot = S.bsdf[S.layer_ids[m.layer_begin + 1]];
+                                                            V3 wo, const float* entry, float mix, St& s) {
+    const DevBsdf top = S.layer[m.layer_begin];
+    const DevBsdf bot = S.layer[m.layer_begin + 1];
     GuidedSample g;
     const float u0 = s.next(), u1 = s.next(), u2 = s.next();
     g.wi_world = guide::cached_mixture_sample(entry, u0, u1, u2);
@@ -130,7 +131,7 @@ __device__ __forceinline__ void coated_walk_weight(const DevScene& S, const DevM
                                                    const LayerEval& e, const float* entry, float mix, V3& f,
                                                    float& pdf) {
     if (e.bounces == 3 && e.out_top && e.pdf > 0.0f && (e.f.x != 0.0f || e.f.y != 0.0f || e.f.z != 0.0f)) {
-        const CoatT1 c = coat_t1(S.bsdf[S.layer_ids[m.layer_begin]], S.bsdf[S.layer_ids[m.layer_begin + 1]], wo, e.wi);
+        const CoatT1 c = coat_t1(S.layer[m.layer_begin], S.layer[m.layer_begin + 1], wo, e.wi);
         f = c.f;
         pdf = mix * guide::cached_mixture_pdf(entry, wi_world) + (1.0f - mix) * c.p;
     } else {
@@ -140,9 +141,10 @@ __device__ __forceinline__ void coated_walk_weight(const DevScene& S, const DevM
 }
 
 // frame: columns u, v (= normal), w.  entry: a lobe-cache entry (guiding.cuh, kCacheEntry floats).
+template <typename St>
 __device__ __forceinline__ GuidedSample guided_sample(const DevScene& S, const DevMaterial& m, const float* frame,
-                                                      V3 wo, const float* entry, float mix, Stream& s) {
-    const DevBsdf b = S.bsdf[S.layer_ids[m.layer_begin]];
+                                                      V3 wo, const float* entry, float mix, St& s) {
+    const DevBsdf b = S.layer[m.layer_begin];
     GuidedSample g;
     if (s.next() < mix) {
         const float u0 = s.next(), u1 = s.next(), u2 = s.next();

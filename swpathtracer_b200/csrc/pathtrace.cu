@@ -8,7 +8,7 @@
 //   k_extend    closest hit for every live slot (traverse*.cuh, the ray casters' traversal)
 //   k_shade     emission, layered BSDF walk, russian roulette and the next ray
 //               (pathtracer.cpp:21-54); surviving paths are appended, warp-aggregated, to the other
-//               buffer; finished paths add their radiance to their scene's image; the last block to
+//               buffer; finished paths add their radiance to their scene's image; the last warp to
 //               finish moves the counters to the next iteration
 //
 // (New paths go behind the live ones, in a kernel of their own: appended by k_shade's lanes in the room of
@@ -61,7 +61,7 @@ struct Counters {
     uint32_t n_alive;               // live slots at the start of the iteration (in the current buffer)
     uint32_t n_next;                // slots appended to the other buffer by k_shade
     uint32_t iterations;
-    uint32_t done;                  // blocks of the running k_shade that have finished
+    uint32_t done;                  // warps of the running k_shade that have finished
     uint32_t rec_count;             // training records written into the current generation
     uint32_t rec_gen;               // generation of the record buffer (bumped when it is consumed)
     uint32_t train_on;              // record training data
@@ -263,7 +263,7 @@ __device__ __forceinline__ uint32_t shade_class(const Wave& W, const PathBuf& cu
     const uint32_t prim = __float_as_uint(__ldg(&hits[i].y));
     if (prim == SPT_MISS) return 0;
     const DevScene& S = W.jobs[__float_as_uint(__ldg(&cur.b[i].w)) >> 16].S;
-    return static_cast<uint32_t>(S.mat[S.prim_mat[prim]].shade_class);
+    return static_cast<uint32_t>(__ldg(&S.mat[surface_of(S, prim).mat].shade_class));
 }
 
 struct ShadeOrder {
@@ -360,14 +360,14 @@ __global__ void __launch_bounds__(256, 3) k_shade(const __grid_constant__ Wave W
                 done = true;
             } else {
                 const float t = h4.x;
-                const bool sphere = J.S.prim_type[prim] == SPT_PRIM_SPHERE;
-                const V3 pos = hit_pos(sphere, o, d, t);
-                const V3 nrm = hit_normal(J.S, prim, h4.z, h4.w, pos);
-                const DevMaterial m = J.S.mat[J.S.prim_mat[prim]];
+                const Surface sf = surface_of(J.S, prim);
+                const V3 pos = hit_pos(sf.type == SPT_PRIM_SPHERE, o, d, t);
+                const V3 nrm = hit_normal(J.S, sf, prim, h4.z, h4.w, pos);
+                const DevMaterial m = J.S.mat[sf.mat];
                 float frame[9];
                 onb_from_normal(nrm, frame);                       // pathtracer.cpp:28-30
                 const V3 wo = normalize(mat_tmul(frame, -d));
-                Stream bs(J.seed, path, static_cast<uint32_t>(depth) + 1u);
+                StreamT<!GUIDED> bs(J.seed, path, static_cast<uint32_t>(depth) + 1u);
                 V3 f, refl, wi, wwi;
                 float pdf;
                 // guided: single-layer materials (guided_sample), and the coated stack from outside
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(256, 3) k_shade(const __grid_constant__ Wave W
                     sampled = true;
                 }
                 if (!sampled) {
-                    const LayerEval e = eval_layered(J.S, m, wo, bs);
+                    const LayerEval e = GUIDED ? eval_layered_call(J.S, m, wo, bs) : eval_layered(J.S, m, wo, bs);
                     f = e.f;
                     refl = e.refl;
                     wi = e.wi;
@@ -470,11 +470,11 @@ __global__ void __launch_bounds__(256, 3) k_shade(const __grid_constant__ Wave W
         }
     }
     }
-    // the last block to finish moves the counters: every block has read them and done its appends
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    // the last warp to finish moves the counters: every warp has read them and done its appends
+    __syncwarp();
+    if (lane == 0) {
         __threadfence();
-        if (atomicAdd(&ctr->done, 1u) == gridDim.x - 1) {
+        if (atomicAdd(&ctr->done, 1u) == gridDim.x * (blockDim.x >> 5) - 1) {
             __threadfence();
             volatile Counters* v = ctr;
             const unsigned long long next = v->next_path + (n - v->n_alive);

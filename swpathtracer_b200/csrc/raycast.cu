@@ -196,12 +196,13 @@ struct TilePixels {
         V3 nrm = v3(0.0f, 0.0f, 0.0f);
         if (found) {
             V3 pos = nrm;   // a sphere's normal needs the hit point: the pixel's ray again
-            if (S.prim_type[prim] == SPT_PRIM_SPHERE) {
+            const Surface sf = surface_of(S, prim);
+            if (sf.type == SPT_PRIM_SPHERE) {
                 V3 o, d;
                 camera_ray(cam, static_cast<float>(i % cam.width) + 0.5f, static_cast<float>(i / cam.width) + 0.5f, o, d);
                 pos = hit_pos(true, o, d, t);
             }
-            nrm = hit_normal(S, prim, u, v, pos);
+            nrm = hit_normal(S, sf, prim, u, v, pos);
         }
         float* q = out + 3ull * i;
         q[0] = nrm.x; q[1] = nrm.y; q[2] = nrm.z;
@@ -254,7 +255,8 @@ __global__ void __launch_bounds__(256) k_raycast(const __grid_constant__ DevScen
                 V3 nrm = v3(0.0f, 0.0f, 0.0f);
                 if (h.found) {
                     const uint32_t prim = slot_prim(S, h.slot);
-                    nrm = hit_normal(S, prim, h.u, h.v, hit_pos(S.prim_type[prim] == SPT_PRIM_SPHERE, o, d, h.t));
+                    const Surface sf = surface_of(S, prim);
+                    nrm = hit_normal(S, sf, prim, h.u, h.v, hit_pos(sf.type == SPT_PRIM_SPHERE, o, d, h.t));
                 }
                 float* q = static_cast<float*>(out) + 3 * idx;
                 q[0] = nrm.x; q[1] = nrm.y; q[2] = nrm.z;
@@ -267,7 +269,8 @@ __global__ void __launch_bounds__(256) k_raycast(const __grid_constant__ DevScen
                 V3 nrm = v3(0.0f, 0.0f, 0.0f);
                 if (h.found) {
                     const uint32_t prim = slot_prim(S, h.slot);
-                    nrm = hit_normal(S, prim, h.u, h.v, hit_pos(S.prim_type[prim] == SPT_PRIM_SPHERE, o, d, h.t));
+                    const Surface sf = surface_of(S, prim);
+                    nrm = hit_normal(S, sf, prim, h.u, h.v, hit_pos(sf.type == SPT_PRIM_SPHERE, o, d, h.t));
                 }
                 float* q = static_cast<float*>(out) + 3 * idx;
                 q[0] = nrm.x; q[1] = nrm.y; q[2] = nrm.z;

@@ -25,16 +25,16 @@ namespace spt {
 //                             + a leaf child's primitive count (0 for an inner child)
 //   leaf[l]                   {first slot, count} of leaf l; leaf_box[l] its box (inside test)
 // ---------------------------------------------------------------------------------------------
-struct DevBsdf {
+struct alignas(16) DevBsdf {
     int type, sampler;
     float r, g, b;        // kd or F0
     float scalar;         // ior or roughness
     float br, bg, bb;     // Lambertian kd / PI (lambertian.cpp:6)
-    float pad;
+    float pad[3];
 };
 
-struct DevMaterial {
-    int layer_begin, layer_count;
+struct alignas(16) DevMaterial {
+    int layer_begin, layer_count;   // its layers, top first: layer[layer_begin ..]
     float er, eg, eb;
     int shade_class;   // what decides the shade kernel's control flow: 1 a layered stack, 2 + type a single BSDF
 };
@@ -44,13 +44,10 @@ struct DevScene {
     const float4* pair;
     const int2* leaf;
     const float* leaf_box;      // 6 floats per leaf
-    const float4* face_normal;  // per primitive (flat triangles)
+    const float4* surface;      // per primitive: face normal (a sphere's centre), material | type << 30
     const float4* smooth_normal;  // 3 per primitive, or null
-    const uint32_t* prim_mat;
-    const uint8_t* prim_type;
-    const DevBsdf* bsdf;
     const DevMaterial* mat;
-    const int* layer_ids;
+    const DevBsdf* layer;       // the BSDFs of every material's layers
     const uint4* wnode;         // 8-wide quantized nodes, 5 x uint4 each (wide_build.h)
     const float4* wtri;         // 3 float4 per primitive in wide-node order: {v0, rank}{e1, prim}{e2, leaf | sphere << 31}
     float root_min[3], root_max[3];
@@ -176,20 +173,27 @@ __device__ __forceinline__ bool sphere_test(V3 c, float radius, V3 o, V3 d, floa
 // Hit position as each primitive's intersect writes it (triangle.cpp:69, sphere.cpp:33).
 __device__ __forceinline__ V3 hit_pos(bool sphere, V3 o, V3 d, float t) { return sphere ? o + t * d : o + d * t; }
 
+// What a hit on a primitive needs of it, in one 16-byte record.
+struct Surface {
+    V3 n;             // face normal, or a sphere's centre
+    uint32_t mat;
+    uint32_t type;
+};
+__device__ __forceinline__ Surface surface_of(const DevScene& S, uint32_t prim) {
+    const float4 f = __ldg(S.surface + prim);
+    const uint32_t w = __float_as_uint(f.w);
+    return Surface{f3v(f), w & 0x3FFFFFFFu, w >> 30};
+}
+
 // Shading normal at a hit (triangle.h:17-21, smooth_triangle.h:11-13, sphere.cpp:34).
-__device__ __forceinline__ V3 hit_normal(const DevScene& S, uint32_t prim, float u, float v, V3 pos) {
-    const uint8_t ty = S.prim_type[prim];
-    if (ty == SPT_PRIM_SPHERE) {
-        // centre is stored in the face-normal slot for spheres
-        float4 c = S.face_normal[prim];
-        return normalize(pos - f3v(c));
-    }
-    if (ty == SPT_PRIM_SMOOTH_TRIANGLE) {
+__device__ __forceinline__ V3 hit_normal(const DevScene& S, const Surface& sf, uint32_t prim, float u, float v, V3 pos) {
+    if (sf.type == SPT_PRIM_SPHERE) return normalize(pos - sf.n);
+    if (sf.type == SPT_PRIM_SMOOTH_TRIANGLE) {
         V3 n0 = f3v(S.smooth_normal[3 * prim]), n1 = f3v(S.smooth_normal[3 * prim + 1]);
         V3 n2 = f3v(S.smooth_normal[3 * prim + 2]);
         return normalize(n0 * ((1.0f - u) - v) + n1 * u + n2 * v);
     }
-    return f3v(S.face_normal[prim]);
+    return sf.n;
 }
 
 // ---- cameras (cameras/pinhole_camera.cpp:14-18, orthographic_camera.cpp:21-25) -----------------
@@ -220,20 +224,26 @@ __device__ __forceinline__ uint4 philox(uint4 c, uint32_t k0, uint32_t k1) {
     return c;
 }
 
+static __device__ __noinline__ uint4 philox_call(uint4 c, uint32_t k0, uint32_t k1) { return philox(c, k0, k1); }
+
 // One sample stream: counter (path index lo, hi, stream id, block); 4 uniforms per block.
-struct Stream {
+// CALL: a block is a call.  Every next() of the layered walk otherwise carries its own copy of the ten
+// rounds, and plain shading waits for instructions (2.5 of its stalls per issue): the layered scene renders
+// in 14.0 instead of 14.1 ms.  Guided shading, whose registers a call would spill, keeps the copies.
+template <bool CALL>
+struct StreamT {
     uint4 ctr;
     uint32_t k0, k1;
     uint4 buf;
     int pos;
-    __device__ __forceinline__ Stream(uint64_t seed, uint64_t path, uint32_t sid)
+    __device__ __forceinline__ StreamT(uint64_t seed, uint64_t path, uint32_t sid)
         : ctr(make_uint4(static_cast<uint32_t>(path), static_cast<uint32_t>(path >> 32), sid, 0u)),
           k0(static_cast<uint32_t>(seed)),
           k1(static_cast<uint32_t>(seed >> 32)),
           pos(4) {}
     __device__ __forceinline__ float next() {
         if (pos == 4) {
-            buf = philox(ctr, k0, k1);
+            buf = CALL ? philox_call(ctr, k0, k1) : philox(ctr, k0, k1);
             ++ctr.w;
             pos = 0;
         }
@@ -242,5 +252,6 @@ struct Stream {
         return static_cast<float>(x >> 8) * (1.0f / 16777216.0f);
     }
 };
+using Stream = StreamT<false>;
 
 }  // namespace spt
