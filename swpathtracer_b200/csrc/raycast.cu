@@ -176,7 +176,7 @@ __device__ __forceinline__ void tile_pixel(uint32_t row_stride, uint32_t& x, uin
 // The depth and normal casters over the 8-wide tree: a warp traces its 8x4 pixels together
 // (traverse_wide.cuh), and the hit's pixel value goes straight out.  What bounds them is the integer unit
 // (64 % of its cycles: permutes, minima and masks of the box tests) and, for a fifth of the time, the longest
-// of the grazing rays.  1920x1080 normals of the 1.31M-triangle mesh take 568 us; each lane testing its own
+// of the grazing rays.  1920x1080 normals of the 1.31M-triangle mesh take 526 us; each lane testing its own
 // triangles took 615, the queries' persistent warps, which refill lanes with other tiles' pixels, 618.
 template <int MODE>
 struct TilePixels {
