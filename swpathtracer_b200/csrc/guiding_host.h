@@ -17,6 +17,15 @@ size_t train_tc_image_bytes();
 void k_mean_weight_launch(const float4* d_rec, uint32_t n, float* out, cudaStream_t s);
 void k_reduce_launch(const float* partial, uint32_t chunks, uint32_t count, float* out, cudaStream_t s);
 
+// Where a gradient call's records come from and its grid gradient goes to host memory: events of the copies'
+// stream, so that the copies overlap the kernels (gradients_tc).
+constexpr uint32_t kHostParts = 4;
+static_assert(kLevels % kHostParts == 0, "whole levels per part");
+struct HostSide {
+    cudaEvent_t arrived[kHostParts];     // part p of the records is on the device
+    cudaEvent_t scattered[kHostParts];   // part p of the grid's levels is final (recorded by gradients_tc)
+};
+
 struct Guide {
     spt_context* ctx = nullptr;
     spt_guide_config cfg{};
@@ -59,6 +68,7 @@ struct Guide {
     uint8_t* touched = nullptr;    // n_cache flags set by guided shading at every entry it reads
     uint32_t* cache_list = nullptr;   // the touched entries of a refresh, then their count at [n_cache]
     bool touched_any = false;      // a guided render has run with this guide (touched is meaningful)
+    HostSide host_side{};          // events of spt_guide_gradients, made on first use
     uint64_t version = 0;          // bumped by every change of the parameters
     uint64_t cache_version = ~0ull;   // the parameter version the cache was last refreshed at
 
@@ -72,7 +82,7 @@ struct Guide {
     spt_status refresh_cache();
     spt_status ensure_train_buffers(uint32_t n);
     spt_status gradients(const float4* d_rec, uint32_t n);
-    spt_status gradients_tc(const float4* d_rec, uint32_t n);
+    spt_status gradients_tc(const float4* d_rec, uint32_t n, const HostSide* host = nullptr);
     spt_status ensure_tc_buffers(uint32_t n);
     spt_status stage_tc();
     spt_status step(const float4* d_rec, uint32_t n, float* loss);
@@ -87,6 +97,10 @@ struct Guide {
         if (cache_list) cudaFree(cache_list);
         for (void* p : train_allocs) cudaFree(p);
         for (void* p : allocations) cudaFree(p);
+        for (uint32_t p = 0; p < kHostParts; ++p) {
+            if (host_side.arrived[p]) cudaEventDestroy(host_side.arrived[p]);
+            if (host_side.scattered[p]) cudaEventDestroy(host_side.scattered[p]);
+        }
     }
 };
 

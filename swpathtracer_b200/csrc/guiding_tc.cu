@@ -66,11 +66,12 @@ __global__ void k_stage_tc(const float* __restrict__ w, unsigned char* __restric
     *reinterpret_cast<__nv_bfloat16*>(img + wb_off(l) + tc::core_offset(k, o, out)) = v;
 }
 
-// feats[16 i + l]: level l's two bf16 features of record i (records: 4 float4, position first).
+// feats[16 i + l]: level l's two bf16 features of the records first .. first + n - 1 (4 float4 each, position
+// first).
 __global__ void __launch_bounds__(256) k_train_inputs(const __grid_constant__ Model M, const float4* __restrict__ rec,
-                                                      uint32_t n, uint32_t* __restrict__ feats) {
-    const uint64_t total = static_cast<uint64_t>(n) * kLevels;
-    for (uint64_t t = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; t < total;
+                                                      uint32_t first, uint32_t n, uint32_t* __restrict__ feats) {
+    const uint64_t begin = static_cast<uint64_t>(first) * kLevels, total = begin + static_cast<uint64_t>(n) * kLevels;
+    for (uint64_t t = begin + blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; t < total;
          t += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         const uint32_t i = static_cast<uint32_t>(t / kLevels), l = static_cast<uint32_t>(t % kLevels);
         const V3 q = normalised_pos(M, f3v(__ldg(rec + 4ull * i)));
@@ -401,15 +402,16 @@ __global__ void __launch_bounds__(kTcRows, 1) k_train_tc(TcIO io) {
     if (warp == 0) tc::tmem_dealloc(tmem, kTmemCols);
 }
 
-// d loss / d grid parameters: each (record, level) spreads its two feature gradients over the cell's
-// 8 corners with their trilinear weights.
+// d loss / d grid parameters of the levels l0 .. l0 + NL - 1: each (record, level) spreads its two feature
+// gradients over the cell's 8 corners with their trilinear weights.
+template <int NL>
 __global__ void __launch_bounds__(256) k_grid_scatter(const __grid_constant__ Model M, const float4* __restrict__ rec,
-                                                      uint32_t n, const float* __restrict__ dx0,
+                                                      uint32_t n, const float* __restrict__ dx0, uint32_t l0,
                                                       float* __restrict__ grid_grad) {
-    const uint64_t total = static_cast<uint64_t>(n) * kLevels;
+    const uint64_t total = static_cast<uint64_t>(n) * NL;
     for (uint64_t t = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; t < total;
          t += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const uint32_t i = static_cast<uint32_t>(t / kLevels), l = static_cast<uint32_t>(t % kLevels);
+        const uint32_t i = static_cast<uint32_t>(t / NL), l = l0 + static_cast<uint32_t>(t % NL);
         const float2 g = __ldg(reinterpret_cast<const float2*>(dx0 + 32ull * i) + l);
         if (g.x == 0.0f && g.y == 0.0f) continue;
         const V3 q = normalised_pos(M, f3v(__ldg(rec + 4ull * i)));
@@ -435,17 +437,24 @@ spt_status Guide::stage_tc() {
 }
 
 // The batch's gradients through the tensor-memory kernels (grid_grad and mlp_grad start at zero).
-spt_status Guide::gradients_tc(const float4* d_rec, uint32_t n) {
+spt_status Guide::gradients_tc(const float4* d_rec, uint32_t n, const HostSide* host) {
     spt_status st = ensure_tc_buffers(n);
     if (st != SPT_OK) return st;
     cudaStream_t s = ctx->stream;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     SPT_CUDA(ctx, cudaMemsetAsync(scalars, 0, 64, s));
+    auto blocks = [&](uint64_t threads) {
+        return static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((threads + 255) / 256, 16ull * sms)));
+    };
+    // a part of the records that has arrived is encoded while the next one is copied in
+    const uint32_t parts = host ? kHostParts : 1, per = (n + parts - 1) / parts;
+    for (uint32_t p = 0; p < parts; ++p) {
+        const uint32_t first = std::min(n, p * per), m = std::min(n, first + per) - first;
+        if (host) SPT_CUDA(ctx, cudaStreamWaitEvent(s, host->arrived[p], 0));
+        if (m) k_train_inputs<<<blocks(static_cast<uint64_t>(m) * kLevels), 256, 0, s>>>(model, d_rec, first, m, tc_feats);
+    }
     k_mean_weight_launch(d_rec, n, scalars, s);
-    const uint64_t pairs = static_cast<uint64_t>(n) * kLevels;
-    const unsigned g_enc = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((pairs + 255) / 256, 16ull * sms)));
-    k_train_inputs<<<g_enc, 256, 0, s>>>(model, d_rec, n, tc_feats);
     TcIO io;
     io.image = tc_image;
     io.rec = d_rec;
@@ -459,7 +468,16 @@ spt_status Guide::gradients_tc(const float4* d_rec, uint32_t n) {
     const uint32_t tiles = (n + kTcRows - 1) / kTcRows;
     const unsigned grid = static_cast<unsigned>(std::max<uint32_t>(1, std::min<uint32_t>(tiles, static_cast<uint32_t>(sms))));
     k_train_tc<<<grid, kTcRows, kSmemTc, s>>>(io);
-    k_grid_scatter<<<g_enc, 256, 0, s>>>(model, d_rec, n, tc_dx0, grid_grad);
+    if (!host) {
+        k_grid_scatter<kLevels><<<blocks(static_cast<uint64_t>(n) * kLevels), 256, 0, s>>>(model, d_rec, n, tc_dx0, 0, grid_grad);
+    } else {
+        // levels in parts, so that a finished one's copy out starts while the next is scattered
+        constexpr int kPart = kLevels / kHostParts;
+        for (uint32_t p = 0; p < kHostParts; ++p) {
+            k_grid_scatter<kPart><<<blocks(static_cast<uint64_t>(n) * kPart), 256, 0, s>>>(model, d_rec, n, tc_dx0, p * kPart, grid_grad);
+            SPT_CUDA(ctx, cudaEventRecord(host->scattered[p], s));
+        }
+    }
     SPT_CUDA(ctx, cudaGetLastError());
     k_reduce_launch(tc_partial, grid, kMlpParams, mlp_grad, s);
     SPT_CUDA(ctx, cudaGetLastError());
