@@ -16,6 +16,12 @@
 // accumulator of the current layer; dW_0..dW_3 (M = 64: out x in) and dW_4^T (in x out) sit at
 // dw_col(l) and keep accumulating until the CTA has no tile left.  In the M = 64 accumulators row r
 // lives in lane 32 * (r / 16) + r % 16.
+//
+// One warp per scheduler works through a tile (the operands of a second tile do not fit in shared
+// memory), so the kernel is bound by the instructions of that warp: 4,000 a tile, about 6 cycles apiece, against
+// 14 MFLOP of contractions.  ReLU and its mask therefore work on packed pairs, a layer has one
+// barrier beside the wait for its MMAs, dW_l runs beside the epilogue of dX_l, and a tile's inputs are
+// loaded during the one before.  2^18 records: 214 -> 177 us (29 GFLOP of contractions).
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -49,7 +55,9 @@ __host__ __device__ constexpr uint32_t x_off(int l) {
     return kImageBytes + (l == 0 ? 0u : 2u * kTcRows * kIn + 2u * kTcRows * kHid * (l - 1));
 }
 constexpr uint32_t kDzOff = x_off(kLayers);
-constexpr uint32_t kBarOff = kDzOff + 2u * kTcRows * kHid;
+constexpr uint32_t kDzBytes = 2u * kTcRows * kHid;
+constexpr uint32_t kBarOff = kDzOff + 2u * kDzBytes;
+__host__ __device__ constexpr uint32_t dz_off(int l) { return kDzOff + (l & 1) * kDzBytes; }
 constexpr uint32_t kSmemTc = kBarOff + 64;
 static_assert(kSmemTc <= 227u * 1024u, "shared memory of k_train_tc");
 static_assert(dw_col(kLayers - 1) + kOut <= kTmemCols, "tensor-memory columns");
@@ -124,6 +132,18 @@ __device__ __forceinline__ float loss_grad_regs(const float (&y)[kOut], V3 wi, f
 #pragma unroll
     for (int k = kOutUsed; k < kOut; ++k) g[k] = 0.0f;
     return -c * logf(q);
+}
+
+// max(x, 0) of two floats as bf16: rounding keeps the sign, so it is done on the packed pair (one
+// instruction for two, and a NaN becomes zero as with fmaxf).
+__device__ __forceinline__ uint32_t relu2(float lo, float hi) {
+    const __nv_bfloat162 r = __hmax2(__floats2bfloat162_rn(lo, hi), __floats2bfloat162_rn(0.0f, 0.0f));
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+// All bits of each half whose bf16 is above zero.
+__device__ __forceinline__ uint32_t positive2(uint32_t x) {
+    return __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&x), __floats2bfloat162_rn(0.0f, 0.0f));
 }
 
 struct TcIO {
@@ -218,31 +238,45 @@ __global__ void __launch_bounds__(kTcRows, 1) k_train_tc(TcIO io) {
             tc::commit(bar);
         }
     };
-    // wait for the committed MMAs; every thread learns whether any wait ran out
-    auto wait_all = [&]() -> bool {
-        const bool mine = tc::mbar_wait(bar, phase, kWaitCycles);
+    // wait for the committed MMAs
+    auto wait = [&] {
+        ok = tc::mbar_wait(bar, phase, kWaitCycles);
         phase ^= 1u;
         tc::fence_after_sync();
-        return __syncthreads_and(mine) != 0;
     };
+    // this thread's shared-memory writes are visible to the next MMAs; every thread learns whether any
+    // wait ran out
+    auto publish = [&]() -> bool {
+        tc::fence_proxy_async();
+        tc::fence_before_sync();
+        return ok = __syncthreads_and(ok) != 0;
+    };
+    // the inputs of a tile's record, loaded while the tile before is worked on
+    uint4 f[4];
+    float4 r1, r2, r3;
+    float weight;
+    auto load = [&](uint32_t row) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) f[c] = make_uint4(0, 0, 0, 0);
+        r1 = r2 = r3 = make_float4(0.f, 0.f, 0.f, 0.f);
+        weight = 0.0f;
+        if (row < io.n) {
+            const uint4* src = reinterpret_cast<const uint4*>(io.feats + 16ull * row);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) f[c] = __ldg(src + c);
+            weight = __ldg(io.rec + 4ull * row).w;
+            r1 = __ldg(io.rec + 4ull * row + 1);
+            r2 = __ldg(io.rec + 4ull * row + 2);
+            r3 = __ldg(io.rec + 4ull * row + 3);
+        }
+    };
+    load(blockIdx.x * kTcRows + tid);
     for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
         const uint32_t row = tile * kTcRows + tid;
         const bool valid = row < io.n;
         // X_0: 32 grid features, normal, wo, zeros
-        float4 r1 = make_float4(0.f, 0.f, 0.f, 0.f), r2 = r1, r3 = r1;
-        float weight = 0.0f;
         {
             unsigned char* x0 = smem + x_off(0);
-            uint4 f[4] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-            if (valid) {
-                const uint4* src = reinterpret_cast<const uint4*>(io.feats + 16ull * row);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) f[c] = __ldg(src + c);
-                weight = __ldg(io.rec + 4ull * row).w;
-                r1 = __ldg(io.rec + 4ull * row + 1);
-                r2 = __ldg(io.rec + 4ull * row + 2);
-                r3 = __ldg(io.rec + 4ull * row + 3);
-            }
 #pragma unroll
             for (int c = 0; c < 4; ++c) put16(x0, tid, 8u * c, kIn, f[c]);
             const uint4 d = valid ? make_uint4(pack2(r1.x, r1.y), pack2(r1.z, r2.x), pack2(r2.y, r2.z), 0u)
@@ -250,9 +284,7 @@ __global__ void __launch_bounds__(kTcRows, 1) k_train_tc(TcIO io) {
             put16(x0, tid, 32, kIn, d);
             put16(x0, tid, 40, kIn, make_uint4(0, 0, 0, 0));
         }
-        tc::fence_proxy_async();
-        tc::fence_before_sync();
-        __syncthreads();
+        if (!publish()) break;
         // ---- forward ----
         float y[kOut];
 #pragma unroll
@@ -262,25 +294,21 @@ __global__ void __launch_bounds__(kTcRows, 1) k_train_tc(TcIO io) {
                 else if (l < kLayers - 1) mma_tile<kHid, kHid>(tmem, sbase + x_off(l), sbase + wf_off(l));
                 else mma_tile<kOut, kHid>(tmem, sbase + x_off(l), sbase + wf_off(l));
             });
-            if (!(ok = wait_all())) break;
+            wait();
             if (l < kLayers - 1) {
                 float v[kHid];
                 ld_row<kHid>(tmem, 0, v);
                 unsigned char* xn = smem + x_off(l + 1);
 #pragma unroll
                 for (int c = 0; c < kHid / 8; ++c) {
-                    const uint4 p = make_uint4(pack2(fmaxf(v[8 * c], 0.f), fmaxf(v[8 * c + 1], 0.f)),
-                                               pack2(fmaxf(v[8 * c + 2], 0.f), fmaxf(v[8 * c + 3], 0.f)),
-                                               pack2(fmaxf(v[8 * c + 4], 0.f), fmaxf(v[8 * c + 5], 0.f)),
-                                               pack2(fmaxf(v[8 * c + 6], 0.f), fmaxf(v[8 * c + 7], 0.f)));
+                    const uint4 p = make_uint4(relu2(v[8 * c], v[8 * c + 1]), relu2(v[8 * c + 2], v[8 * c + 3]),
+                                               relu2(v[8 * c + 4], v[8 * c + 5]), relu2(v[8 * c + 6], v[8 * c + 7]));
                     put16(xn, tid, 8u * c, kHid, p);
                 }
             } else {
                 ld_row<kOut>(tmem, 0, y);
             }
-            tc::fence_proxy_async();
-            tc::fence_before_sync();
-            __syncthreads();
+            if (!publish()) break;
         }
         if (!ok) break;
         // ---- loss and its gradient (mean over the batch) -> dZ_4 ----
@@ -294,54 +322,48 @@ __global__ void __launch_bounds__(kTcRows, 1) k_train_tc(TcIO io) {
 #pragma unroll
                 for (int k = 0; k < kOut; ++k) g[k] = 0.0f;
             }
-            unsigned char* dz = smem + kDzOff;
+            unsigned char* dz = smem + dz_off(kLayers - 1);
 #pragma unroll
             for (int c = 0; c < kOut / 8; ++c)
                 put16(dz, tid, 8u * c, kOut,
                       make_uint4(pack2(g[8 * c], g[8 * c + 1]), pack2(g[8 * c + 2], g[8 * c + 3]),
                                  pack2(g[8 * c + 4], g[8 * c + 5]), pack2(g[8 * c + 6], g[8 * c + 7])));
         }
-        tc::fence_proxy_async();
-        tc::fence_before_sync();
-        __syncthreads();
-        // ---- backward: dX_l = dZ_l W_l (into columns 0..), dW_l += dZ_l^T X_l ----
+        load((tile + gridDim.x) * kTcRows + tid);
+        if (!publish()) break;
+        // ---- backward: dX_l = dZ_l W_l (into columns 0..), dW_l += dZ_l^T X_l.  dW_l is committed with
+        // dX_{l-1}, which nothing waits for before: dZ takes turns between two tiles, and the one dW_l
+        // reads is written again after that commit. ----
         const bool acc = any;
 #pragma unroll
         for (int l = kLayers - 1; l >= 0; --l) {
-            issue([&] {
-                const uint32_t dz = sbase + kDzOff;
-                if (l == kLayers - 1) {
-                    mma_tile<kHid, kOut>(tmem, dz, sbase + wb_off(l));
-                    // dW_4^T [in x out] = X_4^T dZ_4
-                    mma_dw<kOut, kHid>(tmem + dw_col(l), sbase + x_off(l), dz, acc);
-                } else if (l > 0) {
-                    mma_tile<kHid, kHid>(tmem, dz, sbase + wb_off(l));
-                    mma_dw<kHid, kHid>(tmem + dw_col(l), dz, sbase + x_off(l), acc);
-                } else {
-                    mma_tile<kIn, kHid>(tmem, dz, sbase + wb_off(0));
-                    mma_dw<kIn, kHid>(tmem + dw_col(0), dz, sbase + x_off(0), acc);
-                }
-            });
-            if (!(ok = wait_all())) break;
+            const uint32_t dz = sbase + dz_off(l);
+            if (tid == 0) {
+                tc::fence_after_sync();
+                if (l == kLayers - 1) mma_tile<kHid, kOut>(tmem, dz, sbase + wb_off(l));
+                else if (l > 0) mma_tile<kHid, kHid>(tmem, dz, sbase + wb_off(l));
+                else mma_tile<kIn, kHid>(tmem, dz, sbase + wb_off(0));
+                if (l > 0) tc::commit(bar);
+                // dW_4^T [in x out] = X_4^T dZ_4
+                if (l == kLayers - 1) mma_dw<kOut, kHid>(tmem + dw_col(l), sbase + x_off(l), dz, acc);
+                else if (l > 0) mma_dw<kHid, kHid>(tmem + dw_col(l), dz, sbase + x_off(l), acc);
+                else mma_dw<kIn, kHid>(tmem + dw_col(0), dz, sbase + x_off(0), acc);
+                if (l == 0) tc::commit(bar);
+            }
+            wait();
             if (l > 0) {
                 // dZ_{l-1} = dX_l masked by the ReLU of X_l (this thread's row of the X_l tile)
                 float v[kHid];
                 ld_row<kHid>(tmem, 0, v);
                 const unsigned char* xl = smem + x_off(l);
-                unsigned char* dz = smem + kDzOff;
+                unsigned char* dz = smem + dz_off(l - 1);
 #pragma unroll
                 for (int c = 0; c < kHid / 8; ++c) {
                     const uint4 xm = get16(xl, tid, 8u * c, kHid);
                     const uint32_t xw[4] = {xm.x, xm.y, xm.z, xm.w};
                     uint32_t o[4];
 #pragma unroll
-                    for (int h = 0; h < 4; ++h) {
-                        // a bf16 is > 0 when its sign bit is clear and it is not zero
-                        const uint32_t lo = xw[h] & 0xFFFFu, hi = xw[h] >> 16;
-                        const float a = (lo != 0u && !(lo & 0x8000u)) ? v[8 * c + 2 * h] : 0.0f;
-                        const float b = (hi != 0u && !(hi & 0x8000u)) ? v[8 * c + 2 * h + 1] : 0.0f;
-                        o[h] = pack2(a, b);
-                    }
+                    for (int h = 0; h < 4; ++h) o[h] = pack2(v[8 * c + 2 * h], v[8 * c + 2 * h + 1]) & positive2(xw[h]);
                     put16(dz, tid, 8u * c, kHid, make_uint4(o[0], o[1], o[2], o[3]));
                 }
             } else {
@@ -353,9 +375,7 @@ __global__ void __launch_bounds__(kTcRows, 1) k_train_tc(TcIO io) {
                     for (int c = 0; c < 8; ++c) dst[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
                 }
             }
-            tc::fence_proxy_async();
-            tc::fence_before_sync();
-            __syncthreads();
+            if (!publish()) break;
         }
         any = true;
     }
@@ -393,7 +413,7 @@ __global__ void __launch_bounds__(kTcRows, 1) k_train_tc(TcIO io) {
     } else if (tid == 0) {
         atomicOr(io.status, 4u);
         // a wait ran out: give the MMAs in flight one more bounded wait before the columns are freed
-        tc::mbar_wait(bar, phase, kWaitCycles);
+        tc::mbar_wait(bar, phase ^ 1u, kWaitCycles);
     }
     for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xFFFFFFFFu, loss_acc, o);
     if (lane == 0) atomicAdd(io.loss_sum, loss_acc);
