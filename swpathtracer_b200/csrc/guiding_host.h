@@ -19,8 +19,15 @@ void k_reduce_launch(const float* partial, uint32_t chunks, uint32_t count, floa
 
 // Where a gradient call's records come from and its grid gradient goes to host memory: events of the copies'
 // stream, so that the copies overlap the kernels (gradients_tc).
-constexpr uint32_t kHostParts = 4;
+constexpr uint32_t kHostLogParts = 3, kHostParts = 1u << kHostLogParts;
 static_assert(kLevels % kHostParts == 0, "whole levels per part");
+// The parts (a power of two) of n records and of the levels: at least 2^15 records (2 MB, 38 us of copy)
+// each; with fewer the kernels are too short to be worth the extra launches and copies.
+inline uint32_t host_log_parts(uint32_t n) {
+    uint32_t log = 0;
+    while (log < kHostLogParts && n >> (16 + log)) ++log;
+    return log;
+}
 struct HostSide {
     cudaEvent_t arrived[kHostParts];     // part p of the records is on the device
     cudaEvent_t scattered[kHostParts];   // part p of the grid's levels is final (recorded by gradients_tc)

@@ -422,16 +422,15 @@ __global__ void __launch_bounds__(kTcRows, 1) k_train_tc(TcIO io) {
     if (warp == 0) tc::tmem_dealloc(tmem, kTmemCols);
 }
 
-// d loss / d grid parameters of the levels l0 .. l0 + NL - 1: each (record, level) spreads its two feature
+// d loss / d grid parameters of the 2^log_nl levels from l0: each (record, level) spreads its two feature
 // gradients over the cell's 8 corners with their trilinear weights.
-template <int NL>
 __global__ void __launch_bounds__(256) k_grid_scatter(const __grid_constant__ Model M, const float4* __restrict__ rec,
                                                       uint32_t n, const float* __restrict__ dx0, uint32_t l0,
-                                                      float* __restrict__ grid_grad) {
-    const uint64_t total = static_cast<uint64_t>(n) * NL;
+                                                      uint32_t log_nl, float* __restrict__ grid_grad) {
+    const uint64_t total = static_cast<uint64_t>(n) << log_nl;
     for (uint64_t t = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; t < total;
          t += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const uint32_t i = static_cast<uint32_t>(t / NL), l = l0 + static_cast<uint32_t>(t % NL);
+        const uint32_t i = static_cast<uint32_t>(t >> log_nl), l = l0 + (static_cast<uint32_t>(t) & ((1u << log_nl) - 1u));
         const float2 g = __ldg(reinterpret_cast<const float2*>(dx0 + 32ull * i) + l);
         if (g.x == 0.0f && g.y == 0.0f) continue;
         const V3 q = normalised_pos(M, f3v(__ldg(rec + 4ull * i)));
@@ -468,7 +467,7 @@ spt_status Guide::gradients_tc(const float4* d_rec, uint32_t n, const HostSide* 
         return static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((threads + 255) / 256, 16ull * sms)));
     };
     // a part of the records that has arrived is encoded while the next one is copied in
-    const uint32_t parts = host ? kHostParts : 1, per = (n + parts - 1) / parts;
+    const uint32_t log_parts = host ? host_log_parts(n) : 0, parts = 1u << log_parts, per = (n + parts - 1) / parts;
     for (uint32_t p = 0; p < parts; ++p) {
         const uint32_t first = std::min(n, p * per), m = std::min(n, first + per) - first;
         if (host) SPT_CUDA(ctx, cudaStreamWaitEvent(s, host->arrived[p], 0));
@@ -488,15 +487,15 @@ spt_status Guide::gradients_tc(const float4* d_rec, uint32_t n, const HostSide* 
     const uint32_t tiles = (n + kTcRows - 1) / kTcRows;
     const unsigned grid = static_cast<unsigned>(std::max<uint32_t>(1, std::min<uint32_t>(tiles, static_cast<uint32_t>(sms))));
     k_train_tc<<<grid, kTcRows, kSmemTc, s>>>(io);
-    if (!host) {
-        k_grid_scatter<kLevels><<<blocks(static_cast<uint64_t>(n) * kLevels), 256, 0, s>>>(model, d_rec, n, tc_dx0, 0, grid_grad);
-    } else {
-        // levels in parts, so that a finished one's copy out starts while the next is scattered
-        constexpr int kPart = kLevels / kHostParts;
-        for (uint32_t p = 0; p < kHostParts; ++p) {
-            k_grid_scatter<kPart><<<blocks(static_cast<uint64_t>(n) * kPart), 256, 0, s>>>(model, d_rec, n, tc_dx0, p * kPart, grid_grad);
-            SPT_CUDA(ctx, cudaEventRecord(host->scattered[p], s));
-        }
+    // levels in parts, so that a finished one's copy out starts while the next is scattered; the finest
+    // first, because the coarse ones' atomics meet in fewer cells (2^18 records: 85 us for levels 0-3, 49 us
+    // for 12-15) and only the first part is not hidden by copies
+    static_assert(kLevels == 16, "a power of two");
+    const uint32_t log_nl = 4 - log_parts;
+    for (uint32_t p = parts; p-- > 0;) {
+        k_grid_scatter<<<blocks(static_cast<uint64_t>(n) << log_nl), 256, 0, s>>>(model, d_rec, n, tc_dx0, p << log_nl,
+                                                                                  log_nl, grid_grad);
+        if (host) SPT_CUDA(ctx, cudaEventRecord(host->scattered[p], s));
     }
     SPT_CUDA(ctx, cudaGetLastError());
     k_reduce_launch(tc_partial, grid, kMlpParams, mlp_grad, s);
