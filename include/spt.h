@@ -282,7 +282,7 @@ spt_status spt_pathtrace_device(spt_context* ctx, const spt_scene* scene, const 
 
 /* ---- batched rendering and tuning (no reference counterpart) ---------------------------------
  * Many scenes of uneven size and resolution rendered by one wavefront: the camera paths of all jobs
- * share one pool of path slots and the iterations are replayed from one CUDA graph.  Each job's image
+ * share one pool of path slots.  Each job's image
  * is what spt_pathtrace_device would produce for it alone (up to float-add order).  */
 typedef struct spt_tune {
     uint32_t capacity;      /* path slots in the wavefront pool */
@@ -290,8 +290,9 @@ typedef struct spt_tune {
     uint32_t shade_block;   /* threads per block of the shade kernel */
     int32_t traversal;      /* -1 scene default, 0 binary pair nodes, 1 8-wide, 2 8-wide + dynamic fetch */
     uint32_t check_every;   /* guided renders that train: wavefront iterations between the host's looks
-                               at the training records.  Every other render runs its whole loop on the
-                               device (a conditional WHILE node of one CUDA graph) */
+                               at the training records.  Every other render needs no look: its launches
+                               are queued at once when all its paths fit in the pool, else its loop
+                               runs on the device (conditional WHILE nodes of one CUDA graph) */
     uint32_t sort_shading;  /* shade the paths grouped by material class: 0 when a scene has layered
                                materials (their walks diverge most), 1 always, 2 never */
     uint32_t stack;         /* traversal stack depth per lane of the persistent extend kernel: 16, 24 or
@@ -302,7 +303,7 @@ typedef struct spt_tune {
                                0 = a bound from the path count and the 1000-bounce roulette cap */
     uint32_t host_loop;     /* 1: the host replays a graph of two wavefront iterations and reads the
                                counters every check_every iterations (the loop guided training uses)
-                               instead of the device-side WHILE loop; for tools that cannot look into
+                               instead of running without the host; for tools that cannot look into
                                graphs with conditional nodes, such as kernel profilers.  0 = default */
 } spt_tune;
 

@@ -461,7 +461,6 @@ spt_status spt_scene_create(spt_context* ctx, const spt_scene_desc* d, const spt
             });
             S.n_inner = n_inner;
             S.n_leaves = n_leaf;
-            S.n_nodes2 = static_cast<uint32_t>(nn);
             S.root_is_leaf = nodes[0].count ? 1 : 0;
             for (int k = 0; k < 3; ++k) {
                 S.root_min[k] = nodes[0].min[k];

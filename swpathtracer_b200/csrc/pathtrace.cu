@@ -619,9 +619,7 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
         const uint64_t img_elems = 3ull * J.cam.width * J.cam.height;
         if (J.s_begin == 0) SPT_CUDA(ctx, cudaMemsetAsync(J.image, 0, img_elems * sizeof(float), ctx->stream));
     }
-    // Default: the scene's best (8-wide, persistent with dynamic fetch and postponed triangles):
-    // measured 427 vs 405 Mpaths/s on the box workload and 254 vs 233 on the layered one against
-    // the 8-wide tree with one thread per path.
+    // Default: the scene's best, the 8-wide tree with persistent warps and queued triangles.
     if (tune.traversal >= 0 && tune.traversal <= trav) trav = tune.traversal;
     *segments = 0;
     *gpu_ms = 0.0f;

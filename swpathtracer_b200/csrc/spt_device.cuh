@@ -52,7 +52,7 @@ struct DevScene {
     const float4* wtri;         // 3 float4 per primitive in wide-node order: {v0, rank}{e1, prim}{e2, leaf | sphere << 31}
     float root_min[3], root_max[3];
     float bg[3];
-    uint32_t n_prims, n_inner, n_leaves, n_nodes2, n_wnodes;
+    uint32_t n_prims, n_inner, n_leaves, n_wnodes;
     int root_is_leaf;           // the whole scene is one leaf (or no acceleration structure)
     int no_accel;               // NoAccelStructure semantics (no_accel_structure.cpp:9-30)
     int has_spheres;

@@ -142,7 +142,7 @@ __device__ __forceinline__ void wide_node_hits(const uint4* wnode, V3 o, float i
 }
 
 // One candidate triangle/sphere.  Without `exact`, the reference's inside-the-leaf-box test is
-// deferred to the final hit (WideTraversal::finish / closest_hit_wide): a candidate that beats the
+// deferred to the final hit (persistent_trace / closest_hit_wide): a candidate that beats the
 // current best on (t, rank) is kept either way, and if the final hit fails the test the ray is traced
 // again with the test applied to every candidate.  Pruning with a best t that might later be rejected
 // is safe because the final best, once it passes, is the minimum over all candidates with t > 0.
