@@ -203,7 +203,7 @@ def guided_vs_plain(spt, scenes, dev, torch, name, sb, spp, ref_spp, steps, seed
 def path_tracing(spt, scenes, dev, torch, subdiv, renders=7, workload="both", host_loop=False):
     """Path tracing of C0 (box, 256^2, 16 spp, max length 5) and C2 (the layered mesh in the box x3,
     800 x 600, RR after 3, cap 16; 16 spp: the throughput does not depend on spp), each the median of
-    `renders` device-timed renders (spt_pathtrace_device: one launch of the render's graph).  With
+    `renders` device-timed renders (spt_pathtrace_device).  With
     host_loop, the same render as a one-job batch whose loop the host drives (tune.host_loop: a graph
     of two iterations replayed from the host, which kernel profilers can see into)."""
     from swpathtracer_b200 import abi

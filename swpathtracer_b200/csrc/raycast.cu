@@ -226,7 +226,8 @@ __global__ void __launch_bounds__(kTileBlock, 8) k_raycast_wide(const __grid_con
 
 // STATS: the image's statistics (tests and passes of the reference's own traversal, which gives the hit
 // as well).
-template <int MODE, bool STATS>
+// TRAV: the closest-hit traversal without statistics (0 binary, 1 8-wide).
+template <int MODE, bool STATS, int TRAV = 0>
 __global__ void __launch_bounds__(256) k_raycast(const __grid_constant__ DevScene S, const __grid_constant__ DevCamera cam,
                                                  uint32_t row_stride, void* __restrict__ out, StatAcc* stats,
                                                  uint32_t* status) {
@@ -262,7 +263,7 @@ __global__ void __launch_bounds__(256) k_raycast(const __grid_constant__ DevScen
                 q[0] = nrm.x; q[1] = nrm.y; q[2] = nrm.z;
             }
         } else {
-            Hit1 h = trace_closest<0>(S, o, d, status);
+            Hit1 h = trace_closest<TRAV>(S, o, d, status);
             if (MODE == SPT_RAYCAST_DEPTH) {
                 static_cast<float*>(out)[idx] = h.found ? h.t : -1.0f;
             } else {
@@ -435,10 +436,16 @@ static uint32_t row_stride(uint32_t rows) {
 static spt_status launch_raycast(spt_context* ctx, const spt_scene* sc, const DevCamera& cam, int32_t mode, void* d_out,
                                  StatAcc* d_stats, cudaStream_t s) {
     dim3 grid((cam.width + 15) / 16, (cam.height + 15) / 16);
-    // the tiled kernel numbers pixels in 32 bits and rows of tiles in 16; larger images (and statistics, the hit counts and scenes
-    // without a wide tree) take one thread per pixel
-    if (sc->dev.traversal >= 1 && !d_stats && mode != SPT_RAYCAST_COUNT &&
-        static_cast<uint64_t>(cam.width) * cam.height <= 0xFFFFFFFFull && cam.height <= 8u * 65535u) {
+    const uint64_t pixels = static_cast<uint64_t>(cam.width) * cam.height;
+    const bool wide = sc->dev.traversal >= 1 && !d_stats && mode != SPT_RAYCAST_COUNT;
+    // The warp's queue pays once a ray's walk is long or the image too small to hide a lone thread's latency.
+    // Tiled against one thread per pixel, us a normal image: 1,280 triangles 1920x1080 186 / 142, 640x480 55 / 44; 5,120
+    // and 20,480 triangles 1920x1080 221 / 178 and 262 / 227, 320x240 39 / 42 and 47 / 71; 81,920 at 1920x1080 303 / 281,
+    // at 640x480 109 / 135; 327,680 at 1920x1080 386 / 404.
+    const bool short_walks = sc->dev.n_prims <= 2048u || (sc->dev.n_prims <= 131072u && pixels >= 500000u);
+    // the tiled kernel numbers pixels in 32 bits and rows of tiles in 16; larger images (and statistics, the
+    // hit counts and scenes without a wide tree) take one thread per pixel
+    if (wide && !short_walks && pixels <= 0xFFFFFFFFull && cam.height <= 8u * 65535u) {
         const dim3 tiles((cam.width + 15) / 16, (cam.height + 7) / 8);
         auto k = mode == SPT_RAYCAST_NORMAL ? k_raycast_wide<SPT_RAYCAST_NORMAL> : k_raycast_wide<SPT_RAYCAST_DEPTH>;
         k<<<tiles, kTileBlock, 0, s>>>(sc->dev, cam, static_cast<float*>(d_out), ctx->d_status);
@@ -448,6 +455,7 @@ static spt_status launch_raycast(spt_context* ctx, const spt_scene* sc, const De
     auto k = mode == SPT_RAYCAST_NORMAL  ? (d_stats ? k_raycast<SPT_RAYCAST_NORMAL, true> : k_raycast<SPT_RAYCAST_NORMAL, false>)
              : mode == SPT_RAYCAST_DEPTH ? (d_stats ? k_raycast<SPT_RAYCAST_DEPTH, true> : k_raycast<SPT_RAYCAST_DEPTH, false>)
                                          : (d_stats ? k_raycast<SPT_RAYCAST_COUNT, true> : k_raycast<SPT_RAYCAST_COUNT, false>);
+    if (wide) k = mode == SPT_RAYCAST_NORMAL ? k_raycast<SPT_RAYCAST_NORMAL, false, 1> : k_raycast<SPT_RAYCAST_DEPTH, false, 1>;
     k<<<grid, 256, 0, s>>>(sc->dev, cam, row_stride(grid.y), d_out, d_stats, ctx->d_status);
     SPT_CUDA(ctx, cudaGetLastError());
     return SPT_OK;
