@@ -456,11 +456,39 @@ __global__ void k_to_bf16(const float* __restrict__ p, __nv_bfloat16* __restrict
         q[i] = __float2bfloat16_rn(p[i]);
 }
 
-__global__ void k_mean_weight(const float4* __restrict__ rec, uint32_t n, float* __restrict__ out) {
+// The batch's mean weight, the same bits for the same records: every gradient is scaled by its inverse and
+// rounded to bf16, so a mean that followed the warps' order of arrival (float atomics) moved the gradients
+// of one batch by up to 4e-4 (2-norm) from call to call.  The warps leave their shares in `partial`, and
+// the last block to finish (`done`, zero at the start) adds them in a fixed order, in 64 bits.
+constexpr uint32_t kMeanBlocks = 256, kMeanThreads = 256, kMeanWarps = kMeanThreads / 32;
+static_assert(kMeanBlocks * kMeanWarps == kMeanPartials, "one partial per warp");
+__global__ void __launch_bounds__(kMeanThreads) k_mean_weight(const float4* __restrict__ rec, uint32_t n,
+                                                              float* __restrict__ partial, uint32_t* done,
+                                                              float* __restrict__ out) {
+    __shared__ double sum[kMeanWarps];
+    __shared__ bool last;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float s = 0.0f;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += rec[4 * i].w;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += rec[4ull * i].w;
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(out, s / static_cast<float>(n));
+    if (lane == 0) {
+        partial[blockIdx.x * kMeanWarps + warp] = s / static_cast<float>(n);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double t = 0.0;
+    for (uint32_t k = 0; k < kMeanWarps; ++k) t += __ldcg(partial + threadIdx.x * kMeanWarps + k);
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+    if (lane == 0) sum[warp] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (uint32_t w = 1; w < kMeanWarps; ++w) t += sum[w];
+        *out = static_cast<float>(t);
+    }
 }
 
 // deterministic initialisation: grid U(-1e-4, 1e-4), weights N(0, 2/fan_in) (Box-Muller on Philox)
@@ -488,8 +516,9 @@ size_t infer_smem_bytes() {
            kInferWarps * kTileRows * kYld * sizeof(float);
 }
 
-void k_mean_weight_launch(const float4* d_rec, uint32_t n, float* out, cudaStream_t s) {
-    k_mean_weight<<<256, 256, 0, s>>>(d_rec, n, out);
+void Guide::mean_weight(const float4* d_rec, uint32_t n) {
+    k_mean_weight<<<kMeanBlocks, kMeanThreads, 0, ctx->stream>>>(d_rec, n, mean_partial, reinterpret_cast<uint32_t*>(scalars + 2),
+                                                                 scalars);
 }
 
 void k_reduce_launch(const float* partial, uint32_t chunks, uint32_t count, float* out, cudaStream_t s) {
@@ -523,6 +552,7 @@ spt_status Guide::alloc(spt_context* c, const spt_guide_config& cfg_) {
     if ((st = dal(reinterpret_cast<void**>(&mlp_grad), kMlpParams * 4)) != SPT_OK) return st;
     if ((st = dal(reinterpret_cast<void**>(&smem_image), kSmemWeights * 2)) != SPT_OK) return st;
     if ((st = dal(reinterpret_cast<void**>(&scalars), 64)) != SPT_OK) return st;
+    if ((st = dal(reinterpret_cast<void**>(&mean_partial), kMeanPartials * sizeof(float))) != SPT_OK) return st;
     k_init<<<1024, 256, 0, ctx->stream>>>(grid_master, kGridParams, cfg.seed, 0);
     k_init<<<72, 256, 0, ctx->stream>>>(mlp_master, kMlpParams, cfg.seed, 1);
     SPT_CUDA(ctx, cudaGetLastError());
@@ -659,7 +689,7 @@ spt_status Guide::gradients(const float4* d_rec, uint32_t n) {
     cudaStream_t s = ctx->stream;
     // pad n to a multiple of 16 for the tensor-core tiles (padding rows carry zero gradients)
     SPT_CUDA(ctx, cudaMemsetAsync(scalars, 0, 64, s));
-    k_mean_weight<<<256, 256, 0, s>>>(d_rec, n, scalars);
+    mean_weight(d_rec, n);
     TrainIO io;
     io.rec = d_rec;
     io.n = n;

@@ -13,8 +13,7 @@ size_t infer_smem_bytes();
 size_t train_smem_bytes();
 size_t train_tc_smem_bytes();
 size_t train_tc_image_bytes();
-// launchers of guiding.cu's helper kernels, for the tensor-memory training path (guiding_tc.cu)
-void k_mean_weight_launch(const float4* d_rec, uint32_t n, float* out, cudaStream_t s);
+// launcher of guiding.cu's helper kernel, for the tensor-memory training path (guiding_tc.cu)
 void k_reduce_launch(const float* partial, uint32_t chunks, uint32_t count, float* out, cudaStream_t s);
 
 // Where a gradient call's records come from and its grid gradient goes to host memory: events of the copies'
@@ -33,6 +32,8 @@ struct HostSide {
     cudaEvent_t scattered[kHostParts];   // part p of the grid's levels is final (recorded by gradients_tc)
 };
 
+constexpr uint32_t kMeanPartials = 2048;   // shares of a batch's mean weight, one per warp that sums them
+
 struct Guide {
     spt_context* ctx = nullptr;
     spt_guide_config cfg{};
@@ -41,7 +42,8 @@ struct Guide {
     __nv_bfloat16* grid_bf16 = nullptr;
     float *mlp_master = nullptr, *mlp_m = nullptr, *mlp_v = nullptr, *mlp_grad = nullptr;
     __nv_bfloat16* smem_image = nullptr;
-    float* scalars = nullptr;  // [0] mean weight, [1] loss sum
+    float* scalars = nullptr;  // [0] mean weight, [1] loss sum, [2] blocks of k_mean_weight that have finished
+    float* mean_partial = nullptr;
     uint32_t steps = 0;
     std::vector<void*> allocations;
     // training scratch
@@ -88,6 +90,7 @@ struct Guide {
     spt_status ensure_features(uint32_t n);
     spt_status refresh_cache();
     spt_status ensure_train_buffers(uint32_t n);
+    void mean_weight(const float4* d_rec, uint32_t n);   // into scalars[0], with scalars cleared before
     spt_status gradients(const float4* d_rec, uint32_t n);
     spt_status gradients_tc(const float4* d_rec, uint32_t n, const HostSide* host = nullptr);
     spt_status ensure_tc_buffers(uint32_t n);

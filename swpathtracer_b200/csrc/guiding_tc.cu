@@ -484,7 +484,7 @@ spt_status Guide::gradients_tc(const float4* d_rec, uint32_t n, const HostSide* 
         if (host) SPT_CUDA(ctx, cudaStreamWaitEvent(s, host->arrived[p], 0));
         if (m) k_train_inputs<<<blocks(static_cast<uint64_t>(m) * kLevels), 256, 0, s>>>(model, d_rec, first, m, tc_feats);
     }
-    k_mean_weight_launch(d_rec, n, scalars, s);
+    mean_weight(d_rec, n);
     TcIO io;
     io.image = tc_image;
     io.rec = d_rec;
