@@ -590,13 +590,19 @@ spt_status Guide::alloc(spt_context* c, const spt_guide_config& cfg_) {
     return refresh_cache();
 }
 
+// bf16 copies of the current MLP parameters, one per kernel that reads them
+spt_status Guide::stage_mlp() {
+    k_stage<<<(kMlpParams + 255) / 256, 256, 0, ctx->stream>>>(mlp_master, smem_image);
+    SPT_CUDA(ctx, cudaGetLastError());
+    return tc_image ? stage_tc() : SPT_OK;
+}
+
 // bf16 copies of the current master parameters (which have changed: a new parameter version)
 spt_status Guide::refresh() {
     ++version;
-    k_stage<<<(kMlpParams + 255) / 256, 256, 0, ctx->stream>>>(mlp_master, smem_image);
     k_to_bf16<<<4096, 256, 0, ctx->stream>>>(grid_master, grid_bf16, kGridParams);
     SPT_CUDA(ctx, cudaGetLastError());
-    return SPT_OK;
+    return stage_mlp();
 }
 
 spt_status Guide::ensure_features(uint32_t n) {
@@ -729,9 +735,8 @@ spt_status Guide::step(const float4* d_rec, uint32_t n, float* loss) {
     k_adam_sparse<<<4096, 256, 0, ctx->stream>>>(grid_master, grid_m, grid_v, grid_grad, grid_bf16, kGridParams, cfg.lr,
                                                  c1, c2);
     k_adam<<<72, 256, 0, ctx->stream>>>(mlp_master, mlp_m, mlp_v, mlp_grad, nullptr, kMlpParams, cfg.lr, c1, c2);
-    k_stage<<<(kMlpParams + 255) / 256, 256, 0, ctx->stream>>>(mlp_master, smem_image);
     SPT_CUDA(ctx, cudaGetLastError());
-    if (tc_image && (st = stage_tc()) != SPT_OK) return st;
+    if ((st = stage_mlp()) != SPT_OK) return st;
     if (loss) {
         float h[2];
         SPT_CUDA(ctx, cudaMemcpyAsync(h, scalars, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));

@@ -83,6 +83,7 @@ struct Guide {
 
     spt_status alloc(spt_context* c, const spt_guide_config& cfg);
     spt_status refresh();
+    spt_status stage_mlp();
     spt_status infer(const float4* d_in, uint32_t n, float* d_out, cudaStream_t s);
     // inference for a device-side count of samples (at most max_n); usable inside a CUDA graph
     // (ensure_features(max_n) first, outside any stream capture)
