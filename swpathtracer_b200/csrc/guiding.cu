@@ -558,8 +558,6 @@ spt_status Guide::alloc(spt_context* c, const spt_guide_config& cfg_) {
     SPT_CUDA(ctx, cudaGetLastError());
     SPT_CUDA(ctx, cudaFuncSetAttribute(k_infer, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(infer_smem_bytes())));
-    SPT_CUDA(ctx, cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(train_smem_bytes())));
     for (int k = 0; k < 3; ++k) {
         model.lo[k] = cfg.box_min[k];
         const float ext = cfg.box_max[k] - cfg.box_min[k];
@@ -573,9 +571,24 @@ spt_status Guide::alloc(spt_context* c, const spt_guide_config& cfg_) {
     }
     model.grid = grid_bf16;
     model.smem_image = smem_image;
-    // everything a guided render needs is allocated here, so renders and training steps allocate
-    // nothing: the training buffers of one batch, the lobe cache and its inference scratch
-    if ((st = ensure_train_buffers(cfg.batch)) != SPT_OK) return st;
+    // everything a guided render, a training step or a gradient call of up to a batch needs is allocated
+    // here, so that none of them allocates: the buffers of the training path, the room for a batch of
+    // records from host memory, the lobe cache and its inference scratch.  (A first gradient call that
+    // allocated took 4.4 ms with 2^18 records, a repeated one takes 1.8.)
+    if (cfg.train_path == SPT_GUIDE_TRAIN_TCGEN05) {
+        if ((st = ensure_tc_buffers(cfg.batch)) != SPT_OK) return st;
+        for (uint32_t p = 0; p < kHostParts; ++p) {
+            SPT_CUDA(ctx, cudaEventCreateWithFlags(&host_side.arrived[p], cudaEventDisableTiming));
+            SPT_CUDA(ctx, cudaEventCreateWithFlags(&host_side.scattered[p], cudaEventDisableTiming));
+        }
+    } else {
+        SPT_CUDA(ctx, cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           static_cast<int>(train_smem_bytes())));
+        if ((st = ensure_train_buffers(cfg.batch)) != SPT_OK) return st;
+    }
+    void* records;
+    if ((st = scratch(ctx, kRecordScratch, static_cast<size_t>(cfg.batch) * sizeof(spt_guide_record), &records)) != SPT_OK)
+        return st;
     cache_res = cfg.cache_res ? cfg.cache_res : kCacheRes;
     n_cache = cache_res * cache_res * cache_res * 6;
     const uint32_t chunk = std::min(n_cache, kCacheChunk);

@@ -15,7 +15,7 @@ namespace {
 
 spt_status upload_records(spt_context* ctx, const spt_guide_record* recs, uint32_t n, float4** out) {
     void* d;
-    spt_status st = scratch(ctx, 3, static_cast<size_t>(n) * sizeof(spt_guide_record), &d);
+    spt_status st = scratch(ctx, kRecordScratch, static_cast<size_t>(n) * sizeof(spt_guide_record), &d);
     if (st != SPT_OK) return st;
     SPT_CUDA(ctx, cudaMemcpyAsync(d, recs, static_cast<size_t>(n) * sizeof(spt_guide_record), cudaMemcpyHostToDevice,
                                   ctx->stream));
@@ -30,13 +30,9 @@ spt_status upload_records(spt_context* ctx, const spt_guide_record* recs, uint32
 spt_status gradients_overlapped(spt_context* ctx, Guide& G, const spt_guide_record* recs, uint32_t n, float* grid_grad,
                                 float* mlp_grad, float* loss) {
     cudaStream_t s = ctx->stream, copies = ctx->pipe[0];
-    HostSide& H = G.host_side;
-    for (uint32_t p = 0; p < kHostParts; ++p) {
-        if (!H.arrived[p]) SPT_CUDA(ctx, cudaEventCreateWithFlags(&H.arrived[p], cudaEventDisableTiming));
-        if (!H.scattered[p]) SPT_CUDA(ctx, cudaEventCreateWithFlags(&H.scattered[p], cudaEventDisableTiming));
-    }
+    const HostSide& H = G.host_side;
     void* mem;
-    spt_status st = scratch(ctx, 3, static_cast<size_t>(n) * sizeof(spt_guide_record), &mem);
+    spt_status st = scratch(ctx, kRecordScratch, static_cast<size_t>(n) * sizeof(spt_guide_record), &mem);
     if (st != SPT_OK) return st;
     char* d = static_cast<char*>(mem);
     // the copies follow what the context's stream has queued (the buffers' earlier use)

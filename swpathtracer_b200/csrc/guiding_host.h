@@ -32,6 +32,7 @@ struct HostSide {
     cudaEvent_t scattered[kHostParts];   // part p of the grid's levels is final (recorded by gradients_tc)
 };
 
+constexpr int kRecordScratch = 3;          // the context's scratch slot for records from host memory
 constexpr uint32_t kMeanPartials = 2048;   // shares of a batch's mean weight, one per warp that sums them
 
 struct Guide {
@@ -77,7 +78,7 @@ struct Guide {
     uint8_t* touched = nullptr;    // n_cache flags set by guided shading at every entry it reads
     uint32_t* cache_list = nullptr;   // the touched entries of a refresh, then their count at [n_cache]
     bool touched_any = false;      // a guided render has run with this guide (touched is meaningful)
-    HostSide host_side{};          // events of spt_guide_gradients, made on first use
+    HostSide host_side{};          // events of spt_guide_gradients (tcgen05 path)
     uint64_t version = 0;          // bumped by every change of the parameters
     uint64_t cache_version = ~0ull;   // the parameter version the cache was last refreshed at
 

@@ -514,6 +514,7 @@ spt_status Guide::gradients_tc(const float4* d_rec, uint32_t n, const HostSide* 
     return SPT_OK;
 }
 
+// (alloc calls it before the first refresh, which stages the weight image)
 spt_status Guide::ensure_tc_buffers(uint32_t n) {
     if (!tc_image) {
         SPT_CUDA(ctx, cudaMalloc(&tc_image, kImageBytes));
@@ -524,8 +525,6 @@ spt_status Guide::ensure_tc_buffers(uint32_t n) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
         SPT_CUDA(ctx, cudaMalloc(&tc_partial, static_cast<size_t>(sms) * kMlpParams * sizeof(float)));
         allocations.push_back(tc_partial);
-        spt_status st = stage_tc();
-        if (st != SPT_OK) return st;
     }
     if (n <= tc_cap) return SPT_OK;
     if (tc_feats) cudaFree(tc_feats);
