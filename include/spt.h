@@ -371,7 +371,9 @@ spt_status spt_guide_set_params(spt_guide* guide, const float* grid, const float
 /* Mixture for n samples (host arrays): in 12 floats each (pos, 0, normal, 0, wo, 0 as float4s);
  * out 40 floats each: 8 lobes x {mu.xyz, kappa, weight}. */
 spt_status spt_guide_eval(spt_context* ctx, spt_guide* guide, const float* in, uint32_t n, float* out);
-/* Gradients of the mean weighted negative log-likelihood of n records (host), without updating. */
+/* Gradients of the mean weighted negative log-likelihood of n records (host), without updating.  This
+ * call, spt_guide_eval and spt_guide_train run on ctx, which need not be the guide's own context, but must
+ * be on its device; calls on one guide must not overlap in time. */
 spt_status spt_guide_gradients(spt_context* ctx, spt_guide* guide, const spt_guide_record* recs, uint32_t n,
                                float* grid_grad, float* mlp_grad, float* loss);
 /* One Adam step on n records (host). */

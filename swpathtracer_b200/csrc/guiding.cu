@@ -516,9 +516,9 @@ size_t infer_smem_bytes() {
            kInferWarps * kTileRows * kYld * sizeof(float);
 }
 
-void Guide::mean_weight(const float4* d_rec, uint32_t n) {
-    k_mean_weight<<<kMeanBlocks, kMeanThreads, 0, ctx->stream>>>(d_rec, n, mean_partial, reinterpret_cast<uint32_t*>(scalars + 2),
-                                                                 scalars);
+void Guide::mean_weight(const float4* d_rec, uint32_t n, cudaStream_t s) {
+    k_mean_weight<<<kMeanBlocks, kMeanThreads, 0, s>>>(d_rec, n, mean_partial, reinterpret_cast<uint32_t*>(scalars + 2),
+                                                       scalars);
 }
 
 void k_reduce_launch(const float* partial, uint32_t chunks, uint32_t count, float* out, cudaStream_t s) {
@@ -604,10 +604,10 @@ spt_status Guide::alloc(spt_context* c, const spt_guide_config& cfg_) {
 }
 
 // bf16 copies of the current MLP parameters, one per kernel that reads them
-spt_status Guide::stage_mlp() {
-    k_stage<<<(kMlpParams + 255) / 256, 256, 0, ctx->stream>>>(mlp_master, smem_image);
+spt_status Guide::stage_mlp(cudaStream_t s) {
+    k_stage<<<(kMlpParams + 255) / 256, 256, 0, s>>>(mlp_master, smem_image);
     SPT_CUDA(ctx, cudaGetLastError());
-    return tc_image ? stage_tc() : SPT_OK;
+    return tc_image ? stage_tc(s) : SPT_OK;
 }
 
 // bf16 copies of the current master parameters (which have changed: a new parameter version)
@@ -615,7 +615,7 @@ spt_status Guide::refresh() {
     ++version;
     k_to_bf16<<<4096, 256, 0, ctx->stream>>>(grid_master, grid_bf16, kGridParams);
     SPT_CUDA(ctx, cudaGetLastError());
-    return stage_mlp();
+    return stage_mlp(ctx->stream);
 }
 
 spt_status Guide::ensure_features(uint32_t n) {
@@ -699,16 +699,26 @@ spt_status Guide::ensure_train_buffers(uint32_t n) {
     return SPT_OK;
 }
 
-// Gradients of the batch loss (into grid_grad / mlp_grad, which must be zero) and the loss sum: on the
-// tensor-memory kernels (guiding_tc.cu) unless the config asks for the warp-level mma.sync kernels.
-spt_status Guide::gradients(const float4* d_rec, uint32_t n) {
-    if (cfg.train_path == SPT_GUIDE_TRAIN_TCGEN05) return gradients_tc(d_rec, n);
+// grid_grad of zeros for a gradient that is about to be scattered there: the optimiser step leaves it so, a
+// gradient call on its own does not.
+spt_status Guide::clear_gradients(spt_context* c) {
+    if (grid_grad_used) SPT_CUDA(c, cudaMemsetAsync(grid_grad, 0, kGridParams * 4, c->stream));
+    grid_grad_used = true;
+    return SPT_OK;
+}
+
+// Gradients of the batch loss (into grid_grad and mlp_grad) and the loss sum: on the tensor-memory kernels (guiding_tc.cu) unless the config asks for the warp-level mma.sync kernels.
+// Everything runs on the caller's stream, which its records come by; every entry point waits for its own
+// work, so a guide's calls follow one another whichever contexts they come by.
+spt_status Guide::gradients(spt_context* c, const float4* d_rec, uint32_t n) {
+    if (cfg.train_path == SPT_GUIDE_TRAIN_TCGEN05) return gradients_tc(c, d_rec, n);
     spt_status st = ensure_train_buffers(n);
     if (st != SPT_OK) return st;
-    cudaStream_t s = ctx->stream;
+    if ((st = clear_gradients(c)) != SPT_OK) return st;
+    cudaStream_t s = c->stream;
     // pad n to a multiple of 16 for the tensor-core tiles (padding rows carry zero gradients)
-    SPT_CUDA(ctx, cudaMemsetAsync(scalars, 0, 64, s));
-    mean_weight(d_rec, n);
+    SPT_CUDA(c, cudaMemsetAsync(scalars, 0, 64, s));
+    mean_weight(d_rec, n, s);
     TrainIO io;
     io.rec = d_rec;
     io.n = n;
@@ -725,7 +735,7 @@ spt_status Guide::gradients(const float4* d_rec, uint32_t n) {
     const uint32_t tiles = (n + kTileRows - 1) / kTileRows;
     const unsigned grid = static_cast<unsigned>(std::min<uint64_t>((tiles + kWarps - 1) / kWarps, 2ull * sms));
     k_train<<<grid, kWarps * 32, train_smem_bytes(), s>>>(model, io);
-    SPT_CUDA(ctx, cudaGetLastError());
+    SPT_CUDA(c, cudaGetLastError());
     const uint32_t chunks = (io.n_pad + kChunk - 1) / kChunk;
     for (int l = 0; l < kLayers; ++l) {
         const int in = layer_in(l), out = layer_out(l);
@@ -734,26 +744,28 @@ spt_status Guide::gradients(const float4* d_rec, uint32_t n) {
         else k_wgrad<kHid, kHid><<<chunks, 128, 0, s>>>(dzt[l], xt[l], io.n_pad, partial);
         k_reduce<<<(in * out + 255) / 256, 256, 0, s>>>(partial, chunks, in * out, mlp_grad + w_offset(l));
     }
-    SPT_CUDA(ctx, cudaGetLastError());
+    SPT_CUDA(c, cudaGetLastError());
     return SPT_OK;
 }
 
-spt_status Guide::step(const float4* d_rec, uint32_t n, float* loss) {
-    spt_status st = gradients(d_rec, n);
+spt_status Guide::step(spt_context* c, const float4* d_rec, uint32_t n, float* loss) {
+    spt_status st = gradients(c, d_rec, n);
     if (st != SPT_OK) return st;
     ++steps;
     ++version;
     const float c1 = 1.0f - std::pow(0.9f, static_cast<float>(steps));
     const float c2 = 1.0f - std::pow(0.99f, static_cast<float>(steps));
-    k_adam_sparse<<<4096, 256, 0, ctx->stream>>>(grid_master, grid_m, grid_v, grid_grad, grid_bf16, kGridParams, cfg.lr,
-                                                 c1, c2);
-    k_adam<<<72, 256, 0, ctx->stream>>>(mlp_master, mlp_m, mlp_v, mlp_grad, nullptr, kMlpParams, cfg.lr, c1, c2);
-    SPT_CUDA(ctx, cudaGetLastError());
-    if ((st = stage_mlp()) != SPT_OK) return st;
+    k_adam_sparse<<<4096, 256, 0, c->stream>>>(grid_master, grid_m, grid_v, grid_grad, grid_bf16, kGridParams, cfg.lr,
+                                               c1, c2);
+    SPT_CUDA(c, cudaGetLastError());
+    grid_grad_used = false;
+    k_adam<<<72, 256, 0, c->stream>>>(mlp_master, mlp_m, mlp_v, mlp_grad, nullptr, kMlpParams, cfg.lr, c1, c2);
+    SPT_CUDA(c, cudaGetLastError());
+    if ((st = stage_mlp(c->stream)) != SPT_OK) return st;
     if (loss) {
         float h[2];
-        SPT_CUDA(ctx, cudaMemcpyAsync(h, scalars, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-        SPT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        SPT_CUDA(c, cudaMemcpyAsync(h, scalars, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+        SPT_CUDA(c, cudaStreamSynchronize(c->stream));
         *loss = h[1] / static_cast<float>(n);
     }
     return SPT_OK;

@@ -13,6 +13,13 @@ using namespace spt::guide;
 
 namespace {
 
+// A call may come by another context than the guide's own, on the same device.
+spt_status same_device(spt_context* ctx, const spt_guide* guide) {
+    if (guide->g.ctx->device != ctx->device)
+        return fail(ctx, SPT_ERR_INVALID_ARGUMENT, "the guide is on another device");
+    return SPT_OK;
+}
+
 spt_status upload_records(spt_context* ctx, const spt_guide_record* recs, uint32_t n, float4** out) {
     void* d;
     spt_status st = scratch(ctx, kRecordScratch, static_cast<size_t>(n) * sizeof(spt_guide_record), &d);
@@ -38,7 +45,6 @@ spt_status gradients_overlapped(spt_context* ctx, Guide& G, const spt_guide_reco
     // the copies follow what the context's stream has queued (the buffers' earlier use)
     SPT_CUDA(ctx, cudaEventRecord(ctx->ev_pipe[0], s));
     SPT_CUDA(ctx, cudaStreamWaitEvent(copies, ctx->ev_pipe[0], 0));
-    SPT_CUDA(ctx, cudaMemsetAsync(G.grid_grad, 0, kGridParams * 4, s));
     const uint32_t parts = 1u << host_log_parts(n), per = (n + parts - 1) / parts;
     for (uint32_t p = 0; p < parts; ++p) {
         const size_t first = std::min(n, p * per), m = std::min<size_t>(n, first + per) - first;
@@ -47,7 +53,7 @@ spt_status gradients_overlapped(spt_context* ctx, Guide& G, const spt_guide_reco
                                           cudaMemcpyHostToDevice, copies));
         SPT_CUDA(ctx, cudaEventRecord(H.arrived[p], copies));
     }
-    if ((st = G.gradients_tc(reinterpret_cast<const float4*>(d), n, &H)) != SPT_OK) return st;
+    if ((st = G.gradients_tc(ctx, reinterpret_cast<const float4*>(d), n, &H)) != SPT_OK) return st;
     // every kernel is queued: a copy to pageable memory may now hold the host
     if (grid_grad)
         for (uint32_t p = parts; p-- > 0;) {   // the order they are scattered in
@@ -61,7 +67,6 @@ spt_status gradients_overlapped(spt_context* ctx, Guide& G, const spt_guide_reco
     float h[2];
     SPT_CUDA(ctx, cudaMemcpyAsync(h, G.scalars, sizeof(h), cudaMemcpyDeviceToHost, s));
     if ((st = check_status(ctx)) != SPT_OK) return st;
-    SPT_CUDA(ctx, cudaMemsetAsync(G.grid_grad, 0, kGridParams * 4, s));
     if (loss) *loss = h[1] / static_cast<float>(n);
     return SPT_OK;
 }
@@ -125,9 +130,10 @@ spt_status spt_guide_set_params(spt_guide* guide, const float* grid, const float
 spt_status spt_guide_eval(spt_context* ctx, spt_guide* guide, const float* in, uint32_t n, float* out) {
     if (!ctx || !guide || (n && (!in || !out))) return fail(ctx, SPT_ERR_INVALID_ARGUMENT, "NULL argument");
     if (n == 0) return SPT_OK;
+    spt_status st = same_device(ctx, guide);
+    if (st != SPT_OK) return st;
     SPT_CUDA(ctx, cudaSetDevice(ctx->device));
     void *d_in, *d_out;
-    spt_status st;
     if ((st = scratch(ctx, 0, static_cast<size_t>(n) * 48, &d_in)) != SPT_OK) return st;
     if ((st = scratch(ctx, 1, static_cast<size_t>(n) * kOutUsed * 4, &d_out)) != SPT_OK) return st;
     SPT_CUDA(ctx, cudaMemcpyAsync(d_in, in, static_cast<size_t>(n) * 48, cudaMemcpyHostToDevice, ctx->stream));
@@ -140,36 +146,36 @@ spt_status spt_guide_eval(spt_context* ctx, spt_guide* guide, const float* in, u
 spt_status spt_guide_gradients(spt_context* ctx, spt_guide* guide, const spt_guide_record* recs, uint32_t n,
                                float* grid_grad, float* mlp_grad, float* loss) {
     if (!ctx || !guide || !recs || n == 0) return fail(ctx, SPT_ERR_INVALID_ARGUMENT, "NULL argument");
+    spt_status st = same_device(ctx, guide);
+    if (st != SPT_OK) return st;
     SPT_CUDA(ctx, cudaSetDevice(ctx->device));
     Guide& G = guide->g;
     if (G.cfg.train_path == SPT_GUIDE_TRAIN_TCGEN05) {
-        const spt_status st = gradients_overlapped(ctx, G, recs, n, grid_grad, mlp_grad, loss);
+        st = gradients_overlapped(ctx, G, recs, n, grid_grad, mlp_grad, loss);
         if (st != SPT_OK) cudaStreamSynchronize(ctx->pipe[0]);   // no copy is left on the caller's or shared buffers
         return st;
     }
     float4* d;
-    spt_status st = upload_records(ctx, recs, n, &d);
-    if (st != SPT_OK) return st;
-    SPT_CUDA(ctx, cudaMemsetAsync(G.grid_grad, 0, kGridParams * 4, ctx->stream));
-    if ((st = G.gradients(d, n)) != SPT_OK) return st;
+    if ((st = upload_records(ctx, recs, n, &d)) != SPT_OK) return st;
+    if ((st = G.gradients(ctx, d, n)) != SPT_OK) return st;
     if (grid_grad) SPT_CUDA(ctx, cudaMemcpyAsync(grid_grad, G.grid_grad, kGridParams * 4, cudaMemcpyDeviceToHost, ctx->stream));
     if (mlp_grad) SPT_CUDA(ctx, cudaMemcpyAsync(mlp_grad, G.mlp_grad, kMlpParams * 4, cudaMemcpyDeviceToHost, ctx->stream));
     float h[2];
     SPT_CUDA(ctx, cudaMemcpyAsync(h, G.scalars, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     st = check_status(ctx);
     if (st != SPT_OK) return st;
-    SPT_CUDA(ctx, cudaMemsetAsync(G.grid_grad, 0, kGridParams * 4, ctx->stream));
     if (loss) *loss = h[1] / static_cast<float>(n);
     return SPT_OK;
 }
 
 spt_status spt_guide_train(spt_context* ctx, spt_guide* guide, const spt_guide_record* recs, uint32_t n, float* loss) {
     if (!ctx || !guide || !recs || n == 0) return fail(ctx, SPT_ERR_INVALID_ARGUMENT, "NULL argument");
+    spt_status st = same_device(ctx, guide);
+    if (st != SPT_OK) return st;
     SPT_CUDA(ctx, cudaSetDevice(ctx->device));
     float4* d;
-    spt_status st = upload_records(ctx, recs, n, &d);
-    if (st != SPT_OK) return st;
-    if ((st = guide->g.step(d, n, loss)) != SPT_OK) return st;
+    if ((st = upload_records(ctx, recs, n, &d)) != SPT_OK) return st;
+    if ((st = guide->g.step(ctx, d, n, loss)) != SPT_OK) return st;
     return check_status(ctx);
 }
 
@@ -179,7 +185,7 @@ spt_status spt_guide_train_device(spt_context* ctx, spt_guide* guide, const spt_
     if (guide->g.ctx != ctx) return fail(ctx, SPT_ERR_INVALID_ARGUMENT, "the guide belongs to another context");
     SPT_CUDA(ctx, cudaSetDevice(ctx->device));
     SPT_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
-    spt_status st = guide->g.step(reinterpret_cast<const float4*>(d_recs), n, nullptr);
+    spt_status st = guide->g.step(ctx, reinterpret_cast<const float4*>(d_recs), n, nullptr);
     if (st != SPT_OK) return st;
     SPT_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     if ((st = check_status(ctx)) != SPT_OK) return st;   // synchronises the stream

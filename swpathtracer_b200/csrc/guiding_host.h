@@ -46,6 +46,7 @@ struct Guide {
     float* scalars = nullptr;  // [0] mean weight, [1] loss sum, [2] blocks of k_mean_weight that have finished
     float* mean_partial = nullptr;
     uint32_t steps = 0;
+    bool grid_grad_used = false;   // grid_grad holds a gradient that no optimiser step has read (a step clears what it reads)
     std::vector<void*> allocations;
     // training scratch
     __nv_bfloat16* xt[kLayers] = {};
@@ -84,7 +85,7 @@ struct Guide {
 
     spt_status alloc(spt_context* c, const spt_guide_config& cfg);
     spt_status refresh();
-    spt_status stage_mlp();
+    spt_status stage_mlp(cudaStream_t s);
     spt_status infer(const float4* d_in, uint32_t n, float* d_out, cudaStream_t s);
     // inference for a device-side count of samples (at most max_n); usable inside a CUDA graph
     // (ensure_features(max_n) first, outside any stream capture)
@@ -92,12 +93,14 @@ struct Guide {
     spt_status ensure_features(uint32_t n);
     spt_status refresh_cache();
     spt_status ensure_train_buffers(uint32_t n);
-    void mean_weight(const float4* d_rec, uint32_t n);   // into scalars[0], with scalars cleared before
-    spt_status gradients(const float4* d_rec, uint32_t n);
-    spt_status gradients_tc(const float4* d_rec, uint32_t n, const HostSide* host = nullptr);
+    void mean_weight(const float4* d_rec, uint32_t n, cudaStream_t s);   // into scalars[0], with scalars cleared before
+    // c: the context whose stream the work goes to, the guide's own or another on its device
+    spt_status clear_gradients(spt_context* c);
+    spt_status gradients(spt_context* c, const float4* d_rec, uint32_t n);
+    spt_status gradients_tc(spt_context* c, const float4* d_rec, uint32_t n, const HostSide* host = nullptr);
     spt_status ensure_tc_buffers(uint32_t n);
-    spt_status stage_tc();
-    spt_status step(const float4* d_rec, uint32_t n, float* loss);
+    spt_status stage_tc(cudaStream_t s);
+    spt_status step(spt_context* c, const float4* d_rec, uint32_t n, float* loss);
     ~Guide() {
         if (tc_feats) cudaFree(tc_feats);
         if (tc_dx0) cudaFree(tc_dx0);

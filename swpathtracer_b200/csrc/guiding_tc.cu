@@ -460,20 +460,21 @@ __global__ void __launch_bounds__(256) k_grid_scatter(const __grid_constant__ Mo
 size_t train_tc_smem_bytes() { return kSmemTc; }
 size_t train_tc_image_bytes() { return kImageBytes; }
 
-spt_status Guide::stage_tc() {
-    k_stage_tc<<<(kMlpParams + 255) / 256, 256, 0, ctx->stream>>>(mlp_master, tc_image);
+spt_status Guide::stage_tc(cudaStream_t s) {
+    k_stage_tc<<<(kMlpParams + 255) / 256, 256, 0, s>>>(mlp_master, tc_image);
     SPT_CUDA(ctx, cudaGetLastError());
     return SPT_OK;
 }
 
-// The batch's gradients through the tensor-memory kernels (grid_grad and mlp_grad start at zero).
-spt_status Guide::gradients_tc(const float4* d_rec, uint32_t n, const HostSide* host) {
+// The batch's gradients through the tensor-memory kernels.
+spt_status Guide::gradients_tc(spt_context* c, const float4* d_rec, uint32_t n, const HostSide* host) {
     spt_status st = ensure_tc_buffers(n);
     if (st != SPT_OK) return st;
-    cudaStream_t s = ctx->stream;
+    if ((st = clear_gradients(c)) != SPT_OK) return st;
+    cudaStream_t s = c->stream;
     int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    SPT_CUDA(ctx, cudaMemsetAsync(scalars, 0, 64, s));
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    SPT_CUDA(c, cudaMemsetAsync(scalars, 0, 64, s));
     auto blocks = [&](uint64_t threads) {
         return static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((threads + 255) / 256, 16ull * sms)));
     };
@@ -481,10 +482,10 @@ spt_status Guide::gradients_tc(const float4* d_rec, uint32_t n, const HostSide* 
     const uint32_t log_parts = host ? host_log_parts(n) : 0, parts = 1u << log_parts, per = (n + parts - 1) / parts;
     for (uint32_t p = 0; p < parts; ++p) {
         const uint32_t first = std::min(n, p * per), m = std::min(n, first + per) - first;
-        if (host) SPT_CUDA(ctx, cudaStreamWaitEvent(s, host->arrived[p], 0));
+        if (host) SPT_CUDA(c, cudaStreamWaitEvent(s, host->arrived[p], 0));
         if (m) k_train_inputs<<<blocks(static_cast<uint64_t>(m) * kLevels), 256, 0, s>>>(model, d_rec, first, m, tc_feats);
     }
-    mean_weight(d_rec, n);
+    mean_weight(d_rec, n, s);
     TcIO io;
     io.image = tc_image;
     io.rec = d_rec;
@@ -494,7 +495,7 @@ spt_status Guide::gradients_tc(const float4* d_rec, uint32_t n, const HostSide* 
     io.dx0 = tc_dx0;
     io.partial = tc_partial;
     io.loss_sum = scalars + 1;
-    io.status = ctx->d_status;
+    io.status = c->d_status;
     const uint32_t tiles = (n + kTcRows - 1) / kTcRows;
     const unsigned grid = static_cast<unsigned>(std::max<uint32_t>(1, std::min<uint32_t>(tiles, static_cast<uint32_t>(sms))));
     k_train_tc<<<grid, kTcRows, kSmemTc, s>>>(io);
@@ -506,11 +507,11 @@ spt_status Guide::gradients_tc(const float4* d_rec, uint32_t n, const HostSide* 
     for (uint32_t p = parts; p-- > 0;) {
         k_grid_scatter<<<blocks(static_cast<uint64_t>(n) << log_nl), 256, 0, s>>>(model, d_rec, n, tc_dx0, p << log_nl,
                                                                                   log_nl, grid_grad);
-        if (host) SPT_CUDA(ctx, cudaEventRecord(host->scattered[p], s));
+        if (host) SPT_CUDA(c, cudaEventRecord(host->scattered[p], s));
     }
-    SPT_CUDA(ctx, cudaGetLastError());
+    SPT_CUDA(c, cudaGetLastError());
     k_reduce_launch(tc_partial, grid, kMlpParams, mlp_grad, s);
-    SPT_CUDA(ctx, cudaGetLastError());
+    SPT_CUDA(c, cudaGetLastError());
     return SPT_OK;
 }
 

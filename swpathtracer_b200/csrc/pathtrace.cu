@@ -884,7 +884,7 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
             for (uint32_t off = 0; off < n && steps < train_budget; off += batch) {
                 const uint32_t m = std::min(batch, n - off);
                 if (m < batch / 4 && off > 0) break;
-                spt_status s2 = guide->step(G.rec + 4ull * off, m, nullptr);
+                spt_status s2 = guide->step(ctx, G.rec + 4ull * off, m, nullptr);
                 if (s2 != SPT_OK) return s2;
                 ++steps;
             }
