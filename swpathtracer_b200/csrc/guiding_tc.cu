@@ -27,6 +27,7 @@
 #include <algorithm>
 
 #include "guiding_host.h"
+#include "mma_drain.h"
 #include "tc_sm100.cuh"
 
 namespace spt {
@@ -412,8 +413,8 @@ __global__ void __launch_bounds__(kTcRows, 1) k_train_tc(TcIO io) {
         }
     } else if (tid == 0) {
         atomicOr(io.status, 4u);
-        // a wait ran out: give the MMAs in flight one more bounded wait before the columns are freed
-        tc::mbar_wait(bar, phase ^ 1u, kWaitCycles);
+        // a wait ran out; in the backward pass dW_l is then in flight behind the commit that was waited for
+        tc::drain(phase ^ 1u, [&](uint32_t p) { return tc::mbar_wait(bar, p, kWaitCycles); }, [&] { tc::commit(bar); });
     }
     for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xFFFFFFFFu, loss_acc, o);
     if (lane == 0) atomicAdd(io.loss_sum, loss_acc);
