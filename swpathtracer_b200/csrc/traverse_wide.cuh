@@ -75,16 +75,33 @@ __device__ __forceinline__ uint32_t near_first(uint32_t m, uint32_t inv_oct) {
     return m;
 }
 
+// A child is met if its far planes lie behind its near ones by more than rounding can have turned round: the
+// nearest far plane, times 1 + kBoxSlack, not before the farthest near one (after Ize, "Robust BVH Ray
+// Traversal", JCGT 2013).  A hit at t lies between the exact planes, so the computed ones have tmin <=
+// t (1 + 5 x 2^-24) and tmax >= t (1 - 5 x 2^-24), and the hit point that the reference's inside test
+// takes is rounded by 2 x 2^-24 of t on either side: 14 x 2^-24 in all, of which kBoxSlack is more than
+// twice.  (Also of the offset's 255 steps at most, which a converted plane has no margin for: 3 x 2^-24
+// of the node's extent, against the 1e-3 by which the reference's boxes are inflated.)  Without it, rays
+// from far away lost hits: of 2^22 against 1.31M triangles, 2 from 3,000 units, 12 from 6,000, 32 from 8,000;
+// with it none, from 20,000 units either (where the reference's own box test loses hundreds of them).
+// The product takes the place of a subtraction, so it costs no instruction: 2^24 incoherent rays 2.98 ms
+// either way.
+constexpr float kBoxSlack = 1.0f / 524288.0f;   // 2^-19
+__device__ __forceinline__ float boxes_meet(float tmin, float tmax) {   // the sign: not met
+    return __fmaf_rn(tmax, 1.0f + kBoxSlack, -tmin);
+}
+
 // The children of node idx that the ray (o, 1/d) meets before best_t: inner children as near-to-far
 // bits in `hits` (with the node's inner mask and first child), triangles as bits of t_mask from t_base.
 //
 // A child's plane lies at t = (p - o) / d + q 2^e / d, one fused multiply-add.  With 32768 + q in q's
-// place the offset moves by 32768 steps and rounds to within 2^-9 of a step, so the near planes are moved
-// 2^-8 of a step towards the ray's origin and the far planes away from it (both factors, 32768 +- 2^-8,
-// are exact): the tested box contains the quantized one, as that contains the reference's.
+// place the offset (p - o) / d moves by 32768 steps.  Its rounding is then at most 2^-24 of the offset and
+// 2^-9 of a step: the near planes are moved 2^-8 of a step towards the ray's origin and the far planes
+// away from it (both factors, 32768 +- 2^-8, are exact), and what grows with the distance, here and in
+// the offset, 1/d and the multiply-add, at most 5 x 2^-24 of t, is kBoxSlack's (boxes_meet).
 // The box test bounds a visit by its instructions: converting, scaling and comparing 48 planes.  Near
-// and far plane of a child and axis go through one packed multiply-add; the hits gather as the sign bits
-// of tmax - tmin in a mask by slot, which is split into inner children and leaves once; x is converted
+// and far plane of a child and axis go through one packed multiply-add; the hits gather as sign bits
+// (boxes_meet) in a mask by slot, which is split into inner children and leaves once; x is converted
 // and y and z are permuted where the whole warp is in the node step (CONVERT_X).  Against a conversion
 // and a multiply-add per plane and both masks built per child: 2^24 incoherent rays 3.63 against 3.79 ms
 // a call, 300,007 rays 232 against 256 us, the normal caster at 1920x1080 627 against 654 us (641 with
@@ -124,7 +141,7 @@ __device__ __forceinline__ void wide_node_hits(const uint4* wnode, V3 o, float i
         unpack_f2(fma_f2(pack_f2(plane_of<false>(nz0, nz1, j), plane_of<false>(fz0, fz1, j)), s2z, o2z), tnz, tfz);
         const float tmin = fmaxf(max3(tnx, tny, tnz), 0.0f);
         const float tmax = fminf(min3(tfx, tfy, tfz), best_t);
-        missed = __funnelshift_l(__float_as_uint(tmax - tmin), missed, 1);   // the sign of tmax - tmin
+        missed = __funnelshift_l(__float_as_uint(boxes_meet(tmin, tmax)), missed, 1);   // its sign
     }
     const uint32_t met = ~missed & 0xFFu;
     const uint32_t hits = near_first(met & imask, inv_oct);
@@ -596,7 +613,7 @@ __device__ __forceinline__ void trace_last(WarpQueue& Q, Source& src, LaneTrace<
                 const float oz = (__uint_as_float(w0.z) - tr.o.z) * tr.iz;
                 const float tmin = fmaxf(max3(__fmaf_rn(nx, sx, ox), __fmaf_rn(ny, sy, oy), __fmaf_rn(nz, sz, oz)), 0.0f);
                 const float tmax = fminf(min3(__fmaf_rn(fx, sx, ox), __fmaf_rn(fy, sy, oy), __fmaf_rn(fz, sz, oz)), tr.best_t);
-                hit = !(__float_as_uint(tmax - tmin) >> 31);
+                hit = !(__float_as_uint(boxes_meet(tmin, tmax)) >> 31);
                 meta = byte_of(sub < 4 ? w1.z : w1.w, 0u, sub & 3u);
                 imask = w0.w >> 24;
                 tr.g_base = w1.x;
