@@ -789,8 +789,7 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
         // limit's number of them, or until roulette has ended the last path.  They are launched as they
         // are, without a graph: the 64x64 plastic spheres take 166 us instead of 368, the 256x256 box 1.33
         // ms instead of 1.61 (building, instantiating and destroying a graph costs 160 us, and each pass
-        // of its WHILE node adds to its kernels' time).  Under roulette the host looks at the counters
-        // after eight iterations, and after as many again each time it has to go on.
+        // of its WHILE node adds to its kernels' time).
         uint64_t depth_limit = 1;
         bool roulette = false;
         for (const PtJob& J : jobs) {
@@ -798,22 +797,43 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
             roulette |= J.rr != 0;
             depth_limit = std::max<uint64_t>(depth_limit, static_cast<uint64_t>(J.path_length));
         }
-        const bool known = !roulette && depth_limit <= 64 && depth_limit <= max_iter;
+        // (the budget is looked at after every second iteration, as in the device-side loop)
+        const uint64_t budget = (max_iter + 1) & ~1ull;
         SPT_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
         k_generate<<<wave[0].g_gen, 256, 0, ctx->stream>>>(wave[0].W, wave[0].ctr, wave[0].A);
-        for (uint64_t it = 0, stop = known ? depth_limit : 8;;) {
-            // (the budget is looked at after every second iteration, as in the device-side loop)
-            const uint64_t end = known ? stop : std::min<uint64_t>(stop, (max_iter + 1) & ~1ull);
-            for (; it < end; ++it) iteration(wave[0], it);
+        const uint64_t last = roulette ? budget : std::min(depth_limit, budget);   // no path is left after the limit
+        if (!roulette && depth_limit <= 64) {
+            // Paths may all end long before the limit, and an iteration without any takes 10 us: beyond 16
+            // iterations the host looks at the counters of 8, 16 and 32 while as many again run.  A furnace
+            // whose paths end at their second vertex, limit 64: 730 us with every iteration launched,
+            // 245 so; the open box, whose paths live on, 1,608 and 1,628 us (a look's copy takes 8 us).
+            uint64_t it = 0;
+            for (int look = 0;; ++look) {
+                for (const uint64_t end = std::min<uint64_t>(last, 8ull << look); it < end; ++it) iteration(wave[0], it);
+                if (it == last) break;
+                if (last <= 16) continue;
+                SPT_CUDA(ctx, cudaMemcpyAsync(h_head + (look & 1) * kHead, d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost,
+                                              ctx->stream));
+                SPT_CUDA(ctx, cudaEventRecord(ctx->ev_pipe[look & 1], ctx->stream));
+                if (look == 0) continue;
+                SPT_CUDA(ctx, cudaEventSynchronize(ctx->ev_pipe[(look - 1) & 1]));
+                if (counters((look - 1) & 1)->n_alive == 0) break;
+            }
             SPT_CUDA(ctx, cudaGetLastError());
             SPT_CUDA(ctx, cudaMemcpyAsync(h_ctr, d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, ctx->stream));
-            if (known && (st = finalize()) != SPT_OK) return st;
+            if ((st = finalize()) != SPT_OK) return st;
             if ((st = check_status(ctx)) != SPT_OK) return st;   // waits; a stack overflow
-            if (h_ctr->n_alive == 0) break;
-            if (known || it >= max_iter) return fail(ctx, SPT_ERR_TIMEOUT, "a bounded device loop ran out of iterations");
-            stop = 2 * it;
-        }
-        if (!known) {
+            if (h_ctr->n_alive) return fail(ctx, SPT_ERR_TIMEOUT, "a bounded device loop ran out of iterations");
+        } else {
+            // the host waits for eight iterations, and for as many again each time it has to go on
+            for (uint64_t it = 0, stop = 8;; stop = 2 * it) {
+                for (const uint64_t end = std::min(stop, last); it < end; ++it) iteration(wave[0], it);
+                SPT_CUDA(ctx, cudaGetLastError());
+                SPT_CUDA(ctx, cudaMemcpyAsync(h_ctr, d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, ctx->stream));
+                if ((st = check_status(ctx)) != SPT_OK) return st;   // waits; a stack overflow
+                if (h_ctr->n_alive == 0) break;
+                if (it >= last) return fail(ctx, SPT_ERR_TIMEOUT, "a bounded device loop ran out of iterations");
+            }
             if ((st = finalize()) != SPT_OK) return st;
             SPT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         }
