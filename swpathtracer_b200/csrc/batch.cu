@@ -121,7 +121,6 @@ spt_status spt_autotune(spt_context* ctx, const spt_batch_job* jobs, uint32_t n_
         *out = best;
         return SPT_OK;
     }
-    best.traversal = 2;   // what the default (-1) runs, by name: the result says which traversal was timed
     SPT_CUDA(ctx, cudaSetDevice(ctx->device));
     // scratch images for the trials
     size_t total_px = 0;
@@ -139,6 +138,12 @@ spt_status spt_autotune(spt_context* ctx, const spt_batch_job* jobs, uint32_t n_
     }
     std::vector<PtJob> pj;
     if ((st = build_jobs(ctx, trial.data(), n_jobs, imgs.data(), pj)) != SPT_OK) return st;
+    // what the default (-1) runs, by name: the result says which traversal was timed.  A render takes no
+    // higher one than every scene of the batch has (0 for a scene without a tree), so none is tried.
+    best.traversal = 2;
+    for (const PtJob& J : pj)
+        if (J.total) best.traversal = std::min(best.traversal, J.S.traversal);
+    const int32_t highest = best.traversal;
     auto time_of = [&](const spt_tune& t, double& ms_out) -> spt_status {
         uint64_t segs = 0;
         float ms = 0.0f;
@@ -163,7 +168,10 @@ spt_status spt_autotune(spt_context* ctx, const spt_batch_job* jobs, uint32_t n_
         spt_tune round_best = best;
         for (int k = 0; k < n_opt; ++k) {
             spt_tune c = best;
-            if (dim == 0) c.traversal = travs[k];
+            if (dim == 0) {
+                if (travs[k] > highest) continue;
+                c.traversal = travs[k];
+            }
             if (dim == 1) c.capacity = caps[k];
             if (dim == 2) c.shade_block = shades[k];
             if (dim == 3) {
