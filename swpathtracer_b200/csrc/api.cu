@@ -403,11 +403,21 @@ spt_status spt_scene_create(spt_context* ctx, const spt_scene_desc* d, const spt
             any_sphere |= d->prim_type[i] == SPT_PRIM_SPHERE;
         }
         if (any_smooth) smooth.resize(3ull * n);
-        if (d->n_materials > (1u << 30)) return fail(ctx, SPT_ERR_UNSUPPORTED, "more than 2^30 materials");
+        // a primitive names its material in 30 bits (Surface): with more materials than that, the ones that
+        // primitives use are numbered anew
+        std::vector<uint32_t> used;
+        if (d->n_materials > (1u << 30)) {
+            used.assign(d->prim_material, d->prim_material + n);
+            std::sort(used.begin(), used.end());
+            used.erase(std::unique(used.begin(), used.end()), used.end());
+            if (used.size() > (1u << 30)) return fail(ctx, SPT_ERR_UNSUPPORTED, "primitives of more than 2^30 materials");
+        }
         parallel_for(n, [&](size_t a, size_t b) {
             for (size_t i = a; i < b; ++i) {
                 const float* p = d->prim_data + 9ull * i;
-                const float w = bits_f(d->prim_material[i] | static_cast<uint32_t>(d->prim_type[i]) << 30);
+                uint32_t mat = d->prim_material[i];
+                if (!used.empty()) mat = static_cast<uint32_t>(std::lower_bound(used.begin(), used.end(), mat) - used.begin());
+                const float w = bits_f(mat | static_cast<uint32_t>(d->prim_type[i]) << 30);
                 if (d->prim_type[i] == SPT_PRIM_SPHERE) {
                     face[i] = make_float4(p[0], p[1], p[2], w);
                 } else {
@@ -545,17 +555,19 @@ spt_status spt_scene_create(spt_context* ctx, const spt_scene_desc* d, const spt
             o.scalar = b.scalar;
             o.br = b.rgb[0] / kPi; o.bg = b.rgb[1] / kPi; o.bb = b.rgb[2] / kPi;  // lambertian.cpp:6
         }
-        std::vector<DevMaterial> ms(d->n_materials);
-        std::vector<DevBsdf> layers;
+        // each layered BSDF's layers in a row, whatever number of materials share it
+        const uint32_t first_layer = d->n_layered ? d->layered_offsets[0] : 0;
+        std::vector<DevBsdf> layers(d->n_layered ? d->layered_offsets[d->n_layered] - first_layer : 0);
+        for (size_t k = 0; k < layers.size(); ++k) layers[k] = bs[d->layered_bsdf_ids[first_layer + k]];
+        std::vector<DevMaterial> ms(used.empty() ? d->n_materials : used.size());
         bool any_em = false;
-        for (uint32_t i = 0; i < d->n_materials; ++i) {
-            const spt_material& m = d->materials[i];
+        for (size_t i = 0; i < ms.size(); ++i) {
+            const spt_material& m = d->materials[used.empty() ? i : used[i]];
             DevMaterial& o = ms[i];
             std::memset(&o, 0, sizeof(o));
-            o.layer_begin = static_cast<int>(layers.size());
-            for (uint32_t k = d->layered_offsets[m.layered_bsdf]; k < d->layered_offsets[m.layered_bsdf + 1]; ++k)
-                layers.push_back(bs[d->layered_bsdf_ids[k]]);
-            o.layer_count = static_cast<int>(layers.size()) - o.layer_begin;
+            const uint32_t* at = d->layered_offsets + m.layered_bsdf;
+            o.layer_begin = static_cast<int>(at[0] - first_layer);
+            o.layer_count = static_cast<int>(at[1] - at[0]);
             o.er = m.emission[0]; o.eg = m.emission[1]; o.eb = m.emission[2];
             o.shade_class = o.layer_count != 1 ? 1 : 2 + layers[o.layer_begin].type;
             sc->any_layered |= o.layer_count > 1;
