@@ -462,6 +462,7 @@ __device__ __forceinline__ void warp_step(WarpQueue& Q, uint32_t& qhead, uint32_
             tr.last = pos + 1;
         }
         qtail += __popc(found);
+        __syncwarp();   // earlier steps' reservations (votes and reductions order no memory)
         if (lane == 0) Q.tail = qtail;
         __syncwarp();
     }
