@@ -645,15 +645,17 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
     // optimiser steps on the records the paths wrote), or a caller that asks for the host-driven loop
     // (tune.host_loop).
     const bool host_loop = (guide && train_budget > 0) || tune.host_loop != 0;
-    // Every other render whose paths outnumber the pool runs as two waves, each with half the paths and half
-    // the pool, in two branches of one graph: an iteration ends with a few long rays and long walks on a
-    // nearly idle chip, and the other wave's kernels fill it.  The layered scene (3.7 pools) takes 13.65
-    // instead of 14.0 ms, a batch of eight scenes 13.8 instead of 14.35.  Renders within one pool do
-    // not gain (their halves are small, and each has an end of its own): the box takes 1.35 instead of
-    // 1.285 ms.
-    const int waves = !host_loop && total > cap ? 2 : 1;
     bool any_layered = false;
     for (const PtJob& J : jobs) any_layered |= J.layered != 0;
+    // Every other render whose paths outnumber the pool may run as two waves, each with half the paths and
+    // half the pool, in two branches of one graph: an iteration ends with a few long rays and long walks on
+    // a nearly idle chip, and the other wave's kernels fill it.  The second branch costs 200 us to build, and
+    // the walks through layered stacks gain most: one wave against two, ms, the layered scene at 3.4 pools
+    // 10.66 / 10.21, at 13 pools 40.0 / 37.6, at 1.5 pools 4.09 / 4.12; without them the box at 1.5 pools 2.80 /
+    // 3.00, at 13 pools 22.8 / 22.6, at 37 pools 62.5 / 61.5, the 327,680-triangle mesh 2.05 / 2.24, 14.0 / 14.2
+    // and 38.2 / 38.0.  Renders within one pool do not gain either (their halves are small, and each has an
+    // end of its own): the box takes 1.35 instead of 1.285 ms.
+    const int waves = !host_loop && total > cap && total >= (any_layered ? 2 : 32) * cap ? 2 : 1;
     // measured with the block-level order: the box of Lambertian walls and the plain batch scenes level, the
     // guided room 1.46 instead of 1.35 ms
     const bool sort_shading = tune.sort_shading == 1 || (tune.sort_shading == 0 && any_layered);
