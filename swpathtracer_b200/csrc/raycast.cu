@@ -438,11 +438,14 @@ static spt_status launch_raycast(spt_context* ctx, const spt_scene* sc, const De
     dim3 grid((cam.width + 15) / 16, (cam.height + 15) / 16);
     const uint64_t pixels = static_cast<uint64_t>(cam.width) * cam.height;
     const bool wide = sc->dev.traversal >= 1 && !d_stats && mode != SPT_RAYCAST_COUNT;
-    // The warp's queue pays once a ray's walk is long or the image too small to hide a lone thread's latency.
+    // The warp's queue pays once a ray's walk is long, or the image too small to hide a lone thread's latency;
+    // in an image of many pixels to a triangle neighbouring rays share their walks.
     // Tiled against one thread per pixel, us a normal image: 1,280 triangles 1920x1080 186 / 142, 640x480 55 / 44; 5,120
-    // and 20,480 triangles 1920x1080 221 / 178 and 262 / 227, 320x240 39 / 42 and 47 / 71; 81,920 at 1920x1080 303 / 281,
-    // at 640x480 109 / 135; 327,680 at 1920x1080 386 / 404.
-    const bool short_walks = sc->dev.n_prims <= 2048u || (sc->dev.n_prims <= 131072u && pixels >= 500000u);
+    // and 20,480 triangles 1920x1080 225 / 180 and 261 / 225, 320x240 54 / 50 and 59 / 74; 81,920 at 1920x1080 304 /
+    // 282, at 640x480 115 / 133; 327,680 at 1920x1080 382 / 420, 2560x1440 592 / 594, 3840x2160 1,167 / 1,059; 1.31M
+    // at 3840x2160 1,522 / 1,501, 5120x2880 2,505 / 2,421; 5.24M at 5120x2880 3,853 / 4,341, 7680x4320 7,774 / 7,780.
+    const bool short_walks = sc->dev.n_prims <= 2048u || (sc->dev.n_prims <= 131072u && pixels >= 500000u) ||
+                             (sc->dev.n_prims > 131072u && pixels >= 11ull * sc->dev.n_prims);
     // the tiled kernel numbers pixels in 32 bits and rows of tiles in 16; larger images (and statistics, the
     // hit counts and scenes without a wide tree) take one thread per pixel
     if (wide && !short_walks && pixels <= 0xFFFFFFFFull && cam.height <= 8u * 65535u) {
