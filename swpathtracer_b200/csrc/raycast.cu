@@ -418,7 +418,10 @@ spt_status launch_count(spt_context* ctx, const spt_scene* sc, const float* d_ra
 // The stride of the order in which k_raycast starts the rows of tiles: about 0.618 of their number and
 // coprime to it, so every row comes once and neighbours start far apart.  Rows of grazing rays (a
 // silhouette's bottom edge), which the counting traversal follows longest, then do not all start last:
-// 356 against 370 us for the hit counts at 1277x719.  (The tiled kernel above measures the same either way.)
+// 356 against 370 us for the hit counts at 1277x719.  Normals and depths of small scenes gain too (5,120
+// triangles at 1280x720 104 against 115 us); larger ones lose more in L2 than they gain at the end (327,680
+// at 1920x1080 421 against 384 us) and take the rows as they come, as the tiled kernel does, which measures
+// the same either way.
 static uint32_t row_stride(uint32_t rows) {
     uint32_t k = std::max(1u, static_cast<uint32_t>(rows * 0.618));
     auto gcd = [](uint32_t a, uint32_t b) {
@@ -441,11 +444,11 @@ static spt_status launch_raycast(spt_context* ctx, const spt_scene* sc, const De
     // The warp's queue pays once a ray's walk is long, or the image too small to hide a lone thread's latency;
     // in an image of many pixels to a triangle neighbouring rays share their walks.
     // Tiled against one thread per pixel, us a normal image: 1,280 triangles 1920x1080 186 / 142, 640x480 55 / 44; 5,120
-    // and 20,480 triangles 1920x1080 225 / 180 and 261 / 225, 320x240 54 / 50 and 59 / 74; 81,920 at 1920x1080 304 /
-    // 282, at 640x480 115 / 133; 327,680 at 1920x1080 382 / 420, 2560x1440 592 / 594, 3840x2160 1,167 / 1,059; 1.31M
-    // at 3840x2160 1,522 / 1,501, 5120x2880 2,505 / 2,421; 5.24M at 5120x2880 3,853 / 4,341, 7680x4320 7,774 / 7,780.
+    // and 20,480 triangles 1920x1080 227 / 182 and 262 / 225, 320x240 56 / 52 and 60 / 73; 81,920 at 1920x1080 305 /
+    // 278, at 640x480 116 / 130; 327,680 at 1600x900 296 / 322, 1920x1080 380 / 383, 2560x1440 593 / 549; 1.31M at
+    // 2560x1440 803 / 841, 3840x2160 1,525 / 1,438; 5.24M at 5120x2880 3,859 / 3,955, 7680x4320 7,784 / 7,518.
     const bool short_walks = sc->dev.n_prims <= 2048u || (sc->dev.n_prims <= 131072u && pixels >= 500000u) ||
-                             (sc->dev.n_prims > 131072u && pixels >= 11ull * sc->dev.n_prims);
+                             (sc->dev.n_prims > 131072u && pixels >= 6ull * sc->dev.n_prims);
     // the tiled kernel numbers pixels in 32 bits and rows of tiles in 16; larger images (and statistics, the
     // hit counts and scenes without a wide tree) take one thread per pixel
     if (wide && !short_walks && pixels <= 0xFFFFFFFFull && cam.height <= 8u * 65535u) {
@@ -459,7 +462,8 @@ static spt_status launch_raycast(spt_context* ctx, const spt_scene* sc, const De
              : mode == SPT_RAYCAST_DEPTH ? (d_stats ? k_raycast<SPT_RAYCAST_DEPTH, true> : k_raycast<SPT_RAYCAST_DEPTH, false>)
                                          : (d_stats ? k_raycast<SPT_RAYCAST_COUNT, true> : k_raycast<SPT_RAYCAST_COUNT, false>);
     if (wide) k = mode == SPT_RAYCAST_NORMAL ? k_raycast<SPT_RAYCAST_NORMAL, false, 1> : k_raycast<SPT_RAYCAST_DEPTH, false, 1>;
-    k<<<grid, 256, 0, s>>>(sc->dev, cam, row_stride(grid.y), d_out, d_stats, ctx->d_status);
+    const bool spread = mode == SPT_RAYCAST_COUNT || d_stats || sc->dev.n_prims <= 32768u;
+    k<<<grid, 256, 0, s>>>(sc->dev, cam, spread ? row_stride(grid.y) : 1u, d_out, d_stats, ctx->d_status);
     SPT_CUDA(ctx, cudaGetLastError());
     return SPT_OK;
 }
