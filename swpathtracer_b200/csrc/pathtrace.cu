@@ -653,9 +653,11 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
     // the walks through layered stacks gain most: one wave against two, ms, the layered scene at 3.4 pools
     // 10.66 / 10.21, at 13 pools 40.0 / 37.6, at 1.5 pools 4.09 / 4.12; without them the box at 1.5 pools 2.80 /
     // 3.00, at 13 pools 22.8 / 22.6, at 37 pools 62.5 / 61.5, the 327,680-triangle mesh 2.05 / 2.24, 14.0 / 14.2
-    // and 38.2 / 38.0.  Renders within one pool do not gain either (their halves are small, and each has an
+    // and 38.2 / 38.0.  One thread per path (a traversal below 2) has longer ends, and always gains: the
+    // 81,920-triangle mesh at 1.8 pools 3.20 / 2.76, at 7 pools 11.3 / 8.4 (binary tree).  Renders within one pool do not gain either (their halves are small, and each has an
     // end of its own): the box takes 1.35 instead of 1.285 ms.
-    const int waves = !host_loop && total > cap && total >= (any_layered ? 2 : 32) * cap ? 2 : 1;
+    const uint64_t pools = trav < 2 ? 1 : any_layered ? 2 : 32;
+    const int waves = !host_loop && total > cap && total >= pools * cap ? 2 : 1;
     // measured with the block-level order: the box of Lambertian walls and the plain batch scenes level, the
     // guided room 1.46 instead of 1.35 ms
     const bool sort_shading = tune.sort_shading == 1 || (tune.sort_shading == 0 && any_layered);
