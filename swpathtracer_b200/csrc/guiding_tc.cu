@@ -50,8 +50,8 @@ constexpr uint32_t kWHalf = wf_off(kLayers);   // 36,864 bytes
 __host__ __device__ constexpr uint32_t wb_off(int l) { return kWHalf + wf_off(l); }
 constexpr uint32_t kImageBytes = 2 * kWHalf;
 
-// Shared memory: the weight image, the five layer inputs X_0..X_4 (record-major, core layout), one
-// output-gradient tile, the mbarrier and the tensor-memory address.
+// Shared memory: the weight image, the five layer inputs X_0..X_4 (record-major, core layout), two
+// output-gradient tiles, which the layers take in turn, the mbarrier and the tensor-memory address.
 __host__ __device__ constexpr uint32_t x_off(int l) {
     return kImageBytes + (l == 0 ? 0u : 2u * kTcRows * kIn + 2u * kTcRows * kHid * (l - 1));
 }

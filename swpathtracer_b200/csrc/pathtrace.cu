@@ -12,8 +12,7 @@
 //               finish moves the counters to the next iteration
 //
 // (New paths go behind the live ones, in a kernel of their own: appended by k_shade's lanes in the room of
-// ended paths, they mixed camera rays into the warps of bounced ones, and the layered scene took 17.5
-// instead of 16.3 ms.)
+// ended paths, they mixed camera rays into the warps of bounced ones, and the layered scene took 7 % longer.)
 //
 // A batch is a table of jobs (scene + camera + settings); the camera paths of all jobs form one index
 // space, so scenes of very different sizes share the pool, and the iterations are replayed from one
@@ -225,9 +224,9 @@ struct PathRays {
 
 // Persistent extend: lanes take live slots from the iteration's counter as their rays finish.
 // DEPTH: the lane's traversal stack depth (tune.stack); W.stack_limit may hold it lower.  MANY: the
-// batch's jobs are of several scenes (S is the one scene otherwise).  Seven blocks
-// per SM (72 registers): the layered scene renders in 18.2 ms, 18.4 at eight and 19.0 at six; a batch of
-// eight scenes in 18.9, 19.9 at six.
+// batch's jobs are of several scenes (S is the one scene otherwise).  Seven blocks per SM (72 registers): the
+// layered scene renders in 13.7 ms, 13.6 at eight and 14.2 at six; a batch of eight scenes in 13.8, 14.2 at
+// eight and at six.
 template <int DEPTH, bool MANY>
 __global__ void __launch_bounds__(128, 7) k_extend_df(const __grid_constant__ Wave W, const __grid_constant__ DevScene S,
                                                    Counters* __restrict__ ctr, const __grid_constant__ PathBuf cur,
@@ -253,9 +252,8 @@ __device__ __forceinline__ bool rec_live(uint32_t r, uint32_t gen) { return r !=
 // single-layer BSDF.  A block orders a tile of slots by class (a counting sort in shared memory) before it
 // shades them, so its warps take the paths of one class together.  The order is only a permutation of
 // slots: every path computes the same values.  (Counting, scanning and scattering the slots of the whole
-// iteration took three kernels, two passes over the hits and contended global counters: with those and
-// the kernel that moved the counters, the layered scene rendered in 16.6 instead of 16.3 ms, a batch of
-// eight scenes in 17.1 instead of 14.7.)
+// iteration took three kernels, two passes over the hits and contended global counters: with those and a
+// kernel that moved the counters, the layered scene took 2 % longer, a batch of eight scenes 16 %.)
 constexpr uint32_t kShadeClasses = 6;   // miss, layered, 4 single-layer BSDF types
 constexpr uint32_t kShadeTile = 1024;   // slots per tile at most: 32 groups of one warp's width
 
@@ -330,145 +328,145 @@ __global__ void __launch_bounds__(256, 3) k_shade(const __grid_constant__ Wave W
     const uint32_t tile = SORT ? min(kShadeTile, max(1u, (n + gridDim.x * blockDim.x - 1) / (gridDim.x * blockDim.x)) * blockDim.x)
                                : blockDim.x;
     for (uint32_t tbase = blockIdx.x * tile; tbase < n; tbase += gridDim.x * tile) {
-    const uint32_t m = min(tile, n - tbase);
-    if (SORT) order_tile(so, W, cur, hits, tbase, m);
-    // all lanes of a warp iterate together so the append below can be warp-aggregated
-    for (uint32_t off = 0; off < m; off += blockDim.x) {
-        const uint32_t t = off + threadIdx.x;
-        const bool valid = t < m;
-        bool keep = false;
-        float4 wo_o, wo_d, wo_b, wo_l;
-        uint4 rr = make_uint4(kNoRec, kNoRec, kNoRec, kNoRec);
-        if (valid) {
-            const uint32_t i = tbase + (SORT ? so.order[t] : t);   // the slot this lane shades
-            // the slot's last use in this iteration (the buffer is rewritten as the next one's output):
-            // evict-first loads leave L2 to the scene
-            const float4 o4 = __ldcs(cur.o + i), d4 = __ldcs(cur.d + i), b4 = __ldcs(cur.b + i), l4 = __ldcs(cur.l + i),
-                         h4 = __ldcs(hits + i);
-            if (GUIDED && RECORDS) rr = cur.r[i];
-            const uint32_t pix = __float_as_uint(o4.w), sg = __float_as_uint(d4.w);
-            const uint32_t jd = __float_as_uint(b4.w);
-            const int depth = static_cast<int>(jd & 0xFFFFu);
-            const PtJob& J = W.jobs[jd >> 16];
-            const uint64_t path = static_cast<uint64_t>(sg) * J.npix + pix;
-            const V3 o = f3v(o4), d = f3v(d4);
-            V3 beta = f3v(b4), L = f3v(l4);
-            const uint32_t prim = __float_as_uint(h4.y);
-            bool done = false;
-            if (prim == SPT_MISS) {  // pathtracer.cpp:21-26
-                if (depth == 0) L = L + beta * v3(J.S.bg[0], J.S.bg[1], J.S.bg[2]);
-                done = true;
-            } else {
-                const float t = h4.x;
-                const Surface sf = surface_of(J.S, prim);
-                const V3 pos = hit_pos(sf.type == SPT_PRIM_SPHERE, o, d, t);
-                const V3 nrm = hit_normal(J.S, sf, prim, h4.z, h4.w, pos);
-                const DevMaterial m = J.S.mat[sf.mat];
-                float frame[9];
-                onb_from_normal(nrm, frame);                       // pathtracer.cpp:28-30
-                const V3 wo = normalize(mat_tmul(frame, -d));
-                StreamT<!GUIDED> bs(J.seed, path, static_cast<uint32_t>(depth) + 1u);
-                V3 f, refl, wi, wwi;
-                float pdf;
-                // guided: single-layer materials (guided_sample), and the coated stack from outside
-                // (its walk below is the second technique)
-                const bool coat = GUIDED && coated(J.S, m);
-                const uint32_t gi = (GUIDED && static_cast<uint32_t>(depth) < G.depth && guidable(J.S, m) &&
-                                     (!coat || wo.y > 0.0f))
-                                        ? cache_cell(G, pos, nrm)
-                                        : kNoRec;
-                const float* entry = G.cache + static_cast<uint64_t>(guide::kCacheEntry) * (gi != kNoRec ? gi : 0u);
-                if (GUIDED && gi != kNoRec) G.touched[gi] = 1;
-                bool sampled = false;
-                if (GUIDED && gi != kNoRec && (!coat || bs.next() < G.mix)) {
-                    const GuidedSample gs = coat ? coated_guide_sample(J.S, m, frame, wo, entry, G.mix, bs)
-                                                 : guided_sample(J.S, m, frame, wo, entry, G.mix, bs);
-                    f = gs.f;
-                    refl = gs.refl;
-                    wi = gs.wi_local;
-                    wwi = gs.wi_world;
-                    pdf = gs.p;
-                    sampled = true;
-                }
-                if (!sampled) {
-                    const LayerEval e = GUIDED ? eval_layered_call(J.S, m, wo, bs) : eval_layered(J.S, m, wo, bs);
-                    f = e.f;
-                    refl = e.refl;
-                    wi = e.wi;
-                    pdf = e.pdf;
-                    wwi = mat_mul(frame, e.wi);                    // pathtracer.cpp:37-38
-                    if (GUIDED && gi != kNoRec) coated_walk_weight(J.S, m, wo, wwi, e, entry, G.mix, f, pdf);
-                }
-                if (GUIDED && gi != kNoRec && !(pdf > 0.0f)) {
-                    f = v3(0.0f, 0.0f, 0.0f);
-                    pdf = 1.0f;
-                }
-                const V3 no = pos + wwi * 1e-3f;
-                const V3 le = v3(m.er, m.eg, m.eb);
-                if (GUIDED && RECORDS && (le.x != 0.0f || le.y != 0.0f || le.z != 0.0f)) {
-                    // radiance reaching the path's open training records
-                    const V3 add = beta * le;
-                    const uint32_t ids[4] = {rr.x, rr.y, rr.z, rr.w};
-                    for (int k = 0; k < 4; ++k)
-                        if (rec_live(ids[k], rec_gen)) {
-                            float4* sx = G.recx + 2ull * (ids[k] & 0xFFFFFFu) + 1;
-                            const float4 v = *sx;
-                            *sx = make_float4(v.x + add.x, v.y + add.y, v.z + add.z, 0.0f);
-                        }
-                }
-                L = L + beta * le;
-                const float k = fmaxf(fmaxf(refl.x, refl.y), refl.z);
-                if (J.rr && depth >= J.path_length) {              // pathtracer.cpp:43-49
-                    if ((bs.next() < k) && (depth < J.cap)) f = f / k;
-                    else done = true;
-                } else if (J.rr && depth >= J.cap) {
+        const uint32_t count = min(tile, n - tbase);
+        if (SORT) order_tile(so, W, cur, hits, tbase, count);
+        // all lanes of a warp iterate together so the append below can be warp-aggregated
+        for (uint32_t off = 0; off < count; off += blockDim.x) {
+            const uint32_t t = off + threadIdx.x;
+            const bool valid = t < count;
+            bool keep = false;
+            float4 wo_o, wo_d, wo_b, wo_l;
+            uint4 rr = make_uint4(kNoRec, kNoRec, kNoRec, kNoRec);
+            if (valid) {
+                const uint32_t i = tbase + (SORT ? so.order[t] : t);   // the slot this lane shades
+                // the slot's last use in this iteration (the buffer is rewritten as the next one's output):
+                // evict-first loads leave L2 to the scene
+                const float4 o4 = __ldcs(cur.o + i), d4 = __ldcs(cur.d + i), b4 = __ldcs(cur.b + i), l4 = __ldcs(cur.l + i),
+                             h4 = __ldcs(hits + i);
+                if (GUIDED && RECORDS) rr = cur.r[i];
+                const uint32_t pix = __float_as_uint(o4.w), sg = __float_as_uint(d4.w);
+                const uint32_t jd = __float_as_uint(b4.w);
+                const int depth = static_cast<int>(jd & 0xFFFFu);
+                const PtJob& J = W.jobs[jd >> 16];
+                const uint64_t path = static_cast<uint64_t>(sg) * J.npix + pix;
+                const V3 o = f3v(o4), d = f3v(d4);
+                V3 beta = f3v(b4), L = f3v(l4);
+                const uint32_t prim = __float_as_uint(h4.y);
+                bool done = false;
+                if (prim == SPT_MISS) {  // pathtracer.cpp:21-26
+                    if (depth == 0) L = L + beta * v3(J.S.bg[0], J.S.bg[1], J.S.bg[2]);
                     done = true;
-                }
-                if (!done) {
-                    const V3 beta0 = beta;
-                    beta = ((beta * f) * wi.y) / pdf;              // pathtracer.cpp:52-54
-                    if ((beta.x == 0.0f && beta.y == 0.0f && beta.z == 0.0f) ||
-                        (!J.rr && depth + 1 >= J.path_length) ||  // the next trace would return 0
-                        (GUIDED && !(isfinite(beta.x) && isfinite(beta.y) && isfinite(beta.z)))) {
-                        done = true;
-                    } else {
-                        if (GUIDED && RECORDS && gi != kNoRec && train_on) {
-                            const uint32_t r = atomicAdd(&ctr->rec_count, 1u);
-                            if (r < G.rec_cap) {
-                                G.rec[4ull * r] = make_float4(pos.x, pos.y, pos.z, 0.0f);
-                                G.rec[4ull * r + 1] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
-                                G.rec[4ull * r + 2] = make_float4(-d.x, -d.y, -d.z, 0.0f);
-                                G.rec[4ull * r + 3] = make_float4(wwi.x, wwi.y, wwi.z, 0.0f);
-                                G.recx[2ull * r] = make_float4(beta0.x, beta0.y, beta0.z, 0.0f);
-                                G.recx[2ull * r + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                                rr = make_uint4(((rec_gen & 0xFFu) << 24) | r, rr.x, rr.y, rr.z);
+                } else {
+                    const float t = h4.x;
+                    const Surface sf = surface_of(J.S, prim);
+                    const V3 pos = hit_pos(sf.type == SPT_PRIM_SPHERE, o, d, t);
+                    const V3 nrm = hit_normal(J.S, sf, prim, h4.z, h4.w, pos);
+                    const DevMaterial m = J.S.mat[sf.mat];
+                    float frame[9];
+                    onb_from_normal(nrm, frame);                       // pathtracer.cpp:28-30
+                    const V3 wo = normalize(mat_tmul(frame, -d));
+                    StreamT<!GUIDED> bs(J.seed, path, static_cast<uint32_t>(depth) + 1u);
+                    V3 f, refl, wi, wwi;
+                    float pdf;
+                    // guided: single-layer materials (guided_sample), and the coated stack from outside
+                    // (its walk below is the second technique)
+                    const bool coat = GUIDED && coated(J.S, m);
+                    const uint32_t gi = (GUIDED && static_cast<uint32_t>(depth) < G.depth && guidable(J.S, m) &&
+                                         (!coat || wo.y > 0.0f))
+                                            ? cache_cell(G, pos, nrm)
+                                            : kNoRec;
+                    const float* entry = G.cache + static_cast<uint64_t>(guide::kCacheEntry) * (gi != kNoRec ? gi : 0u);
+                    if (GUIDED && gi != kNoRec) G.touched[gi] = 1;
+                    bool sampled = false;
+                    if (GUIDED && gi != kNoRec && (!coat || bs.next() < G.mix)) {
+                        const GuidedSample gs = coat ? coated_guide_sample(J.S, m, frame, wo, entry, G.mix, bs)
+                                                     : guided_sample(J.S, m, frame, wo, entry, G.mix, bs);
+                        f = gs.f;
+                        refl = gs.refl;
+                        wi = gs.wi_local;
+                        wwi = gs.wi_world;
+                        pdf = gs.p;
+                        sampled = true;
+                    }
+                    if (!sampled) {
+                        const LayerEval e = GUIDED ? eval_layered_call(J.S, m, wo, bs) : eval_layered(J.S, m, wo, bs);
+                        f = e.f;
+                        refl = e.refl;
+                        wi = e.wi;
+                        pdf = e.pdf;
+                        wwi = mat_mul(frame, e.wi);                    // pathtracer.cpp:37-38
+                        if (GUIDED && gi != kNoRec) coated_walk_weight(J.S, m, wo, wwi, e, entry, G.mix, f, pdf);
+                    }
+                    if (GUIDED && gi != kNoRec && !(pdf > 0.0f)) {
+                        f = v3(0.0f, 0.0f, 0.0f);
+                        pdf = 1.0f;
+                    }
+                    const V3 no = pos + wwi * 1e-3f;
+                    const V3 le = v3(m.er, m.eg, m.eb);
+                    if (GUIDED && RECORDS && (le.x != 0.0f || le.y != 0.0f || le.z != 0.0f)) {
+                        // radiance reaching the path's open training records
+                        const V3 add = beta * le;
+                        const uint32_t ids[4] = {rr.x, rr.y, rr.z, rr.w};
+                        for (int k = 0; k < 4; ++k)
+                            if (rec_live(ids[k], rec_gen)) {
+                                float4* sx = G.recx + 2ull * (ids[k] & 0xFFFFFFu) + 1;
+                                const float4 v = *sx;
+                                *sx = make_float4(v.x + add.x, v.y + add.y, v.z + add.z, 0.0f);
                             }
+                    }
+                    L = L + beta * le;
+                    const float k = fmaxf(fmaxf(refl.x, refl.y), refl.z);
+                    if (J.rr && depth >= J.path_length) {              // pathtracer.cpp:43-49
+                        if ((bs.next() < k) && (depth < J.cap)) f = f / k;
+                        else done = true;
+                    } else if (J.rr && depth >= J.cap) {
+                        done = true;
+                    }
+                    if (!done) {
+                        const V3 beta0 = beta;
+                        beta = ((beta * f) * wi.y) / pdf;              // pathtracer.cpp:52-54
+                        if ((beta.x == 0.0f && beta.y == 0.0f && beta.z == 0.0f) ||
+                            (!J.rr && depth + 1 >= J.path_length) ||  // the next trace would return 0
+                            (GUIDED && !(isfinite(beta.x) && isfinite(beta.y) && isfinite(beta.z)))) {
+                            done = true;
+                        } else {
+                            if (GUIDED && RECORDS && gi != kNoRec && train_on) {
+                                const uint32_t r = atomicAdd(&ctr->rec_count, 1u);
+                                if (r < G.rec_cap) {
+                                    G.rec[4ull * r] = make_float4(pos.x, pos.y, pos.z, 0.0f);
+                                    G.rec[4ull * r + 1] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
+                                    G.rec[4ull * r + 2] = make_float4(-d.x, -d.y, -d.z, 0.0f);
+                                    G.rec[4ull * r + 3] = make_float4(wwi.x, wwi.y, wwi.z, 0.0f);
+                                    G.recx[2ull * r] = make_float4(beta0.x, beta0.y, beta0.z, 0.0f);
+                                    G.recx[2ull * r + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                                    rr = make_uint4(((rec_gen & 0xFFu) << 24) | r, rr.x, rr.y, rr.z);
+                                }
+                            }
+                            keep = true;
+                            wo_o = make_float4(no.x, no.y, no.z, o4.w);
+                            wo_d = make_float4(wwi.x, wwi.y, wwi.z, d4.w);
+                            wo_b = make_float4(beta.x, beta.y, beta.z, __uint_as_float(jd + 1u));
+                            wo_l = make_float4(L.x, L.y, L.z, 0.0f);
                         }
-                        keep = true;
-                        wo_o = make_float4(no.x, no.y, no.z, o4.w);
-                        wo_d = make_float4(wwi.x, wwi.y, wwi.z, d4.w);
-                        wo_b = make_float4(beta.x, beta.y, beta.z, __uint_as_float(jd + 1u));
-                        wo_l = make_float4(L.x, L.y, L.z, 0.0f);
                     }
                 }
+                if (done) splat(J, pix, L);
             }
-            if (done) splat(J, pix, L);
-        }
-        const unsigned kept = __ballot_sync(0xFFFFFFFFu, keep);
-        if (kept) {
-            uint32_t first = 0;
-            if (lane == 0) first = atomicAdd(&ctr->n_next, static_cast<uint32_t>(__popc(kept)));
-            first = __shfl_sync(0xFFFFFFFFu, first, 0);
-            if (keep) {
-                const uint32_t slot = first + __popc(kept & ((1u << lane) - 1u));
-                nxt.o[slot] = wo_o;
-                nxt.d[slot] = wo_d;
-                nxt.b[slot] = wo_b;
-                nxt.l[slot] = wo_l;
-                if (GUIDED && RECORDS) nxt.r[slot] = rr;
+            const unsigned kept = __ballot_sync(0xFFFFFFFFu, keep);
+            if (kept) {
+                uint32_t first = 0;
+                if (lane == 0) first = atomicAdd(&ctr->n_next, static_cast<uint32_t>(__popc(kept)));
+                first = __shfl_sync(0xFFFFFFFFu, first, 0);
+                if (keep) {
+                    const uint32_t slot = first + __popc(kept & ((1u << lane) - 1u));
+                    nxt.o[slot] = wo_o;
+                    nxt.d[slot] = wo_d;
+                    nxt.b[slot] = wo_b;
+                    nxt.l[slot] = wo_l;
+                    if (GUIDED && RECORDS) nxt.r[slot] = rr;
+                }
             }
         }
-    }
     }
     // the last warp to finish moves the counters: every warp has read them and done its appends
     __syncwarp();
@@ -654,12 +652,13 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
     // 10.66 / 10.21, at 13 pools 40.0 / 37.6, at 1.5 pools 4.09 / 4.12; without them the box at 1.5 pools 2.80 /
     // 3.00, at 13 pools 22.8 / 22.6, at 37 pools 62.5 / 61.5, the 327,680-triangle mesh 2.05 / 2.24, 14.0 / 14.2
     // and 38.2 / 38.0.  One thread per path (a traversal below 2) has longer ends, and always gains: the
-    // 81,920-triangle mesh at 1.8 pools 3.20 / 2.76, at 7 pools 11.3 / 8.4 (binary tree).  Renders within one pool do not gain either (their halves are small, and each has an
-    // end of its own): the box takes 1.35 instead of 1.285 ms.
+    // 81,920-triangle mesh at 1.8 pools 3.20 / 2.76, at 7 pools 11.3 / 8.4 (binary tree).  Renders within one
+    // pool do not gain (their halves are small, and each has an end of its own): the box takes 1.35 instead of
+    // 1.285 ms.
     const uint64_t pools = trav < 2 ? 1 : any_layered ? 2 : 32;
     const int waves = !host_loop && total > cap && total >= pools * cap ? 2 : 1;
     // measured with the block-level order: the box of Lambertian walls and the plain batch scenes level, the
-    // guided room 1.46 instead of 1.35 ms
+    // guided room 8 % slower with it, the layered scene 5.12 ms at 640x480 and 9 samples instead of 5.49
     const bool sort_shading = tune.sort_shading == 1 || (tune.sort_shading == 0 && any_layered);
     {   // counters and job table, neighbours in memory, in one copy
         std::vector<char> head(2 * kHead + job_bytes, 0);
@@ -791,9 +790,9 @@ spt_status render_jobs(spt_context* ctx, std::vector<PtJob>& jobs, const spt_tun
     if (total <= cap && !host_loop) {
         // The pool holds every path from the start, so the render is a handful of iterations: the depth
         // limit's number of them, or until roulette has ended the last path.  They are launched as they
-        // are, without a graph: the 64x64 plastic spheres take 166 us instead of 368, the 256x256 box 1.33
-        // ms instead of 1.61 (building, instantiating and destroying a graph costs 160 us, and each pass
-        // of its WHILE node adds to its kernels' time).
+        // are, without a graph: building, instantiating and destroying one costs 160 us (the 64x64 plastic
+        // spheres take 175 us a call without), and each pass of its WHILE node adds to its kernels' time
+        // (the 256x256 box took 1.33 ms instead of 1.61).
         uint64_t depth_limit = 1;
         bool roulette = false;
         for (const PtJob& J : jobs) {

@@ -60,8 +60,8 @@ struct RayBatch {
 };
 
 // Persistent variant: wide traversal, lanes refilled from a global ray counter (traverse_wide.cuh).
-// 8 blocks of 128 per SM (at most 64 registers): when the triangle queue came in, 2^24 incoherent rays
-// took 3.86 ms a call at 8 blocks, 4.22 at 10 (48 registers, 150 bytes spilled), 3.93 at 7, 4.22 at 6.
+// 8 blocks of 128 per SM (at most 64 registers): 2^24 incoherent rays take 3.01 ms a call at 8 blocks, 3.13 at 7, 3.37 at
+// 6, 3.32 at 9 and 3.42 at 10, where the ray's state spills.
 template <int STRIDE>
 __global__ void __launch_bounds__(kBlock, 8) k_intersect_df(const __grid_constant__ DevScene S,
                                                          const float* __restrict__ rays, uint32_t n,

@@ -153,7 +153,8 @@ __device__ __forceinline__ void count_leaf(const DevScene& S, uint32_t first, ui
 // A step visits a pair node: both children's boxes and, for a leaf child, its primitive count, in one
 // 64-byte record.  What bounds the traversal is its chain of dependent node loads and the boxes' slab
 // tests; a step per box, from the tree's own 32-byte nodes, and with the primitives tested for counts
-// that do not need them, took 1268 us on 1277x719 camera rays against 1.31M triangles, where this takes 369.
+// that do not need them, took 1268 us on 1277x719 camera rays against 1.31M triangles, where this takes 350 (369
+// before the rows of tiles were spread, raycast.cu).
 template <int STACK, bool FULL>
 __device__ __forceinline__ Hit1 count_traverse(const DevScene& S, V3 o, V3 d, CountOut& c, uint32_t* overflow) {
     Hit1 h;

@@ -102,10 +102,10 @@ __device__ __forceinline__ float boxes_meet(float tmin, float tmax) {   // the s
 // The box test bounds a visit by its instructions: converting, scaling and comparing 48 planes.  Near
 // and far plane of a child and axis go through one packed multiply-add; the hits gather as sign bits
 // (boxes_meet) in a mask by slot, which is split into inner children and leaves once; x is converted
-// and y and z are permuted where the whole warp is in the node step (CONVERT_X).  Against a conversion
-// and a multiply-add per plane and both masks built per child: 2^24 incoherent rays 3.63 against 3.79 ms
-// a call, 300,007 rays 232 against 256 us, the normal caster at 1920x1080 627 against 654 us (641 with
-// CONVERT_X), the layered path tracing 18.6 against 19.2 ms.
+// and y and z are permuted where the whole warp is in the node step (CONVERT_X: 2^24 incoherent rays 3.01 ms a
+// call, 3.07 with x permuted too, the normal caster at 1920x1080 557 and 574 us, the layered path tracing 13.7
+// and 13.8 ms).  When this test came in, a conversion and a multiply-add per plane and both masks built per
+// child took 4 % more on the 2^24 rays, 10 % on 300,007.
 template <bool CONVERT_X>
 __device__ __forceinline__ void wide_node_hits(const uint4* wnode, V3 o, float ix, float iy, float iz,
                                                uint32_t inv_oct, uint32_t idx, float best_t, uint32_t& g_base,
@@ -263,9 +263,9 @@ __device__ __forceinline__ Hit1 closest_hit_wide(const DevScene& S, V3 o, V3 d, 
 // (t, rank) over every candidate and a stale best t is only ever too large.  And a ray is finished
 // when it has no node left and its last queued triangle has been tested.
 //
-// On 2^24 incoherent rays against 1.31M triangles the call (order and gather included) takes 3.00 ms, and
-// took 5.14 with each lane testing its own triangles and the lane's state in local memory; 300,007
-// rays 199 against 372 us; path tracing the layered scene 16.6 against 26.9 ms a render.
+// On 2^24 incoherent rays against 1.31M triangles the call (order and gather included) takes 2.99 ms, and
+// took 5.14 with each lane testing its own triangles and the lane's state in local memory; 300,007 rays
+// 161 against 372 us.
 //
 // The per-lane node stack is an array of its own, not a member of the lane's state: a dynamically
 // indexed member keeps the whole struct around it in local memory (the kernels that had it so read
@@ -284,8 +284,8 @@ struct WarpQueue {
     uint32_t pool, pool_end;            // the warp's rays in hand
     uint32_t chunk, first;              // rays per chunk, and the first ray the counter hands out
 };
-// A warp stops waiting for 32 triangles once this many lanes have nothing else to do (4, 8 and 16 measure
-// alike).
+// A warp stops waiting for 32 triangles once this many lanes have nothing else to do (queries and paths
+// measure alike at 4, 8 and 16).
 constexpr int kWait = 8;
 constexpr unsigned long long kNoHitKey = 0x7F800000FFFFFFFFull;   // t = +inf, any rank
 
@@ -435,9 +435,9 @@ __device__ __forceinline__ void warp_step(WarpQueue& Q, uint32_t& qhead, uint32_
     if (tr.walking()) tr.visit(W.wnode, stack, limit, status, t_base, t_mask);
     // Room for all of them (31 at most are left over, and a step finds 15 on average): each lane reserves a
     // run of places with one shared-memory atomic and fills it.  Otherwise one triangle per lane at a
-    // time, with tests in between.  (Appending one per lane at a time throughout took six rounds of
-    // ballots a step: 3.44 against 3.00 ms a call on 2^24 incoherent rays, the layered path tracing 18.3
-    // against 16.6 ms.)
+    // time, with tests in between.  (Appending one per lane at a time throughout takes six rounds of
+    // ballots a step: 3.38 against 3.01 ms a call on 2^24 incoherent rays, the layered path tracing 14.8
+    // against 13.7 ms, the normal caster 648 against 557 us.)
     const uint32_t mine = __popc(t_mask), all = __reduce_add_sync(0xFFFFFFFFu, mine);
     if (!all) return;
     const unsigned long long first =
@@ -480,12 +480,12 @@ __device__ __forceinline__ void test_rest(WarpQueue& Q, uint32_t& qhead, uint32_
 // Persistent warps with dynamic ray fetch (after Aila & Laine, "Understanding the Efficiency of Ray
 // Traversal on GPUs", HPG 2009): a lane whose ray is finished takes the next ray at once instead of
 // idling until the warp's longest ray ends.  Ray indices come from a warp-local pool refilled `chunk`
-// at a time from one global counter, so the counter sees one atomic per chunk.  32 rays per chunk:
-// against 64 it measured +0.6 % on the ordered incoherent queries and +4.6 % / +8.2 % on the box and
-// layered path tracing (a shorter tail, and the ordered neighbours stay together); 128 lost 3 %.
+// at a time from one global counter, so the counter sees one atomic per chunk.  2^24 rays take 3.08 / 3.01 / 3.00
+// / 3.06 ms at 16 / 32 / 64 / 128 rays per chunk, the layered path tracing 13.6 / 13.7 / 14.5 / 15.9, the box 1.29
+// / 1.30 / 1.34 / 1.45 (a shorter tail, and the ordered neighbours stay together).
 constexpr uint32_t kChunk = 32;
 // Lanes are served (hit stored, next ray taken) once this many wait, or no lane is busy: the branch runs
-// with the waiting lanes only.  2^24 rays take 3.79 / 3.63 / 3.51 / 3.53 / 3.64 ms at 2 / 4 / 8 / 12 / 16.
+// with the waiting lanes only.  2^24 rays take 3.30 / 3.14 / 3.01 / 3.01 / 3.10 ms at 2 / 4 / 8 / 12 / 16.
 constexpr int kRefill = 8;
 
 // source: load(i, o, d) fetches ray i (and, for a kernel of many scenes, the lane's scene), move(from)
@@ -514,9 +514,10 @@ __device__ __forceinline__ bool settle(const WarpQueue& Q, Source& src, const La
 // The warp's last rays, four at most: eight lanes to a ray, one child of its node each.  A lone lane's
 // visit is a chain of some 400 instructions, most of them the eight children's box tests one after the
 // other; a batch of a few rays per warp, and the end of any batch, waits for such chains (the longest
-// ray of 1,000 incoherent ones visits 88 nodes: alone it took 80 us, here 55).  300,007 rays against
-// 1.31M triangles take 156 us instead of 199, the layered path tracing 15.6 ms instead of 16.4.  The lanes of a group hold copies of the ray's state;
-// the first of them, its leader, keeps the node stack, the best hit and the queue entries' name.
+// ray of 1,000 incoherent ones visits 88 nodes: alone it took 80 us, here 55).  300,007 rays against 1.31M
+// triangles take 161 us instead of 203, the layered path tracing 13.7 ms instead of 14.6, the normal caster 557
+// us instead of 581.  The lanes of a group hold copies of the ray's state; the first of them, its leader,
+// keeps the node stack, the best hit and the queue entries' name.
 constexpr int kLast = 4;
 template <int DEPTH, bool COUNT, typename Source>
 __device__ __forceinline__ void trace_last(WarpQueue& Q, Source& src, LaneTrace<DEPTH, COUNT>& tr, uint2 (&stack)[DEPTH],
