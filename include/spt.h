@@ -290,8 +290,8 @@ typedef struct spt_tune {
     uint32_t shade_block;   /* threads per block of the shade kernel */
     int32_t traversal;      /* -1 scene default, 0 binary pair nodes, 1 8-wide, 2 8-wide + dynamic fetch */
     uint32_t check_every;   /* guided renders that train: wavefront iterations between the host's looks
-                               at the training records.  Every other render needs no look: its launches
-                               are queued at once when all its paths fit in the pool, else its loop
+                               at the training records.  Every other render's iterations are launched
+                               as they are when all its paths fit in the pool, else its loop
                                runs on the device (conditional WHILE nodes of one CUDA graph) */
     uint32_t sort_shading;  /* shade the paths grouped by material class: 0 when a scene has layered
                                materials (their walks diverge most), 1 always, 2 never */

@@ -15,8 +15,9 @@
 // ended paths, they mixed camera rays into the warps of bounced ones, and the layered scene took 7 % longer.)
 //
 // A batch is a table of jobs (scene + camera + settings); the camera paths of all jobs form one index
-// space, so scenes of very different sizes share the pool, and the iterations are replayed from one
-// CUDA graph.  A single-scene render is a batch of one.
+// space, so scenes of very different sizes share the pool; the iterations are launched as they are where
+// the pool holds every path, and loop in one CUDA graph where it does not.  A single-scene render is a batch
+// of one.
 //
 // Random numbers: Philox-4x32-10 keyed by the job's seed, counter (path index, stream, block), stream 0
 // for the pixel sample and stream depth+1 for the BSDF walk and roulette at that depth.  The path
